@@ -12,14 +12,15 @@
 // region:
 //   header words 0..5 : 24 one-byte tags, slot s at word s / 4, byte s % 4; 0 = free, 0xFF = being written
 //   header word 6     : handle of the body (item of slot 0)
-//   header word 7     : header id of the next slab in the bucket's chain, 0 = end (header 0 is unused)
+//   header word 7     : header id of the next slab in the bucket's chain, 0 = end (header 0 is unused),
+//                       kLinking = end, a slab is being appended
 //   body              : 24 items of k words at a stride of k rounded up to a multiple of 4 (slot s at body + s*stride)
 // A probe reads one 32-byte header sector per slab plus the candidate item. Headers are dense (a
 // table's headers are about a tenth of its bytes), so the headers a lookup stream touches stay in
 // the 126 MB L2 while the items it compares are read once; the reference interleaves a 10-word
 // header with each slab's items (compact_acceleration_hash_table.h:519-541). The first slab of each
 // bucket is allocated with the table (HASH_TABLE_STORE_SLABS_IN_TABLE, gpu_hash_table_base.h:30-49);
-// overflow slabs come from bump allocators over the two regions and are linked at the chain's tail.
+// overflow slabs come from bump allocators over the two regions and are appended at the chain's tail.
 //
 // Free list (DynamicSlabAllocator::free, dynamic_slab_alloc.h:187-208, and the sweep's unlinking of
 // empty slabs, gpu_hash_table_base.cu:265-281,320-336): garbage collection unlinks every overflow
@@ -41,6 +42,7 @@ namespace svdag {
 
 constexpr uint32_t kNone = 0xFFFFFFFFu; // empty child / missing handle
 constexpr uint32_t kEnd = 0u; // end of a slab chain
+constexpr uint32_t kLinking = 0xFFFFFFFFu; // end of a slab chain whose next slab is being allocated
 constexpr uint32_t kFillMarker = 0xFFFFFF00u; // SVO child "canonical fully-filled node of material m" = kFillMarker | m
 constexpr uint32_t kUnitWords = 4; // a handle counts 16-byte units
 constexpr unsigned long long kMaxItemWords = (unsigned long long)kUnitWords * 0xFFFFFF00ull - 64; // item region limit (just under 64 GiB)
@@ -497,6 +499,7 @@ __device__ __forceinline__ uint32_t first_slab(const DevTable& t, uint32_t cls, 
 }
 
 constexpr uint32_t kFreeListTries = 64; // pops that lose this many races fall back to the bump allocator
+constexpr uint32_t kLinkTries = 1u << 18; // bound on waiting for another thread's slab (tens of milliseconds)
 
 // Takes a slab off the free list of size class `cls`; kNone when the list is empty (or contended).
 // The head's version count changes with every pop and push, so a pop whose head is stale fails its
@@ -604,38 +607,40 @@ __device__ __forceinline__ uint32_t alloc_slab(const Grp<G>& g, const DevDag& d,
     return id;
 }
 
-// Links `fresh` behind `slab`; returns the slab that follows `slab` afterwards (ours or a racer's).
-__device__ __forceinline__ uint32_t link_slab(const DevDag& d, uint32_t slab, uint32_t fresh)
-{
-    const uint32_t prev = atomicCAS(slab_ptr(d, slab) + 7, kEnd, fresh);
-    return prev == kEnd ? fresh : prev;
-}
-
-// An overflow slab allocated by a group that lost the race to link it; it may only be linked into a
-// chain of the same size class later.
-struct Spare {
-    uint32_t slab = kNone;
-    uint32_t k = 0;
-};
-
-// Gives an unused spare back: a level table's goes on its class's free list; other tables' spares
-// stay allocated (their space comes back when the bump pointers are rewound or never).
+// The slab after `slab` in its chain, appended when the chain ends there. The thread that turns the
+// end mark into kLinking allocates; the others wait for the link it publishes (bounded, then
+// SVDAG_ERR_TIMEOUT). A full bucket so costs one slab and one trip to the allocator however many
+// threads find it full at once: when every one of them allocated and all but one gave their slab
+// back, a tile of a depth-13 scene build spent 22 ms of one merge launch on the free list's head word.
+// kNone when a region is full (SVDAG_ERR_OOM) or the wait ran out.
 template <int G>
-__device__ __forceinline__ void release_spare(const Grp<G>& g, const DevDag& d, const DevTable& t, Spare& spare)
+__device__ __forceinline__ uint32_t append_slab(const Grp<G>& g, const DevDag& d, const DevTable& t, uint32_t slab, uint32_t k)
 {
-    if (spare.slab != kNone && t.recycle && g.lane == 0)
-        push_free_chain(d, spare.k - 2u, spare.slab, spare.slab, 1);
-    spare.slab = kNone;
-}
-// A spare of another size class than `k` is released before a new one is allocated.
-template <int G>
-__device__ __forceinline__ void take_spare(const Grp<G>& g, const DevDag& d, const DevTable& t, Spare& spare, uint32_t k)
-{
-    if (spare.slab == kNone || spare.k != k) {
-        release_spare<G>(g, d, t, spare);
-        spare.slab = alloc_slab<G>(g, d, k, t.recycle);
-        spare.k = k;
+    uint32_t* link = slab_ptr(d, slab) + 7;
+    uint32_t next = 0;
+    if (g.lane == 0)
+        next = atomicCAS(link, kEnd, kLinking);
+    next = g.bcast(next, 0);
+    if (next == kEnd) {
+        const uint32_t fresh = alloc_slab<G>(g, d, k, t.recycle); // its header and body are visible to other SMs
+        if (g.lane == 0)
+            atomicExch(link, fresh == kNone ? kEnd : fresh);
+        g.sync();
+        return fresh;
     }
+    if (g.lane == 0) {
+        for (uint32_t tries = 0; next == kLinking; ++tries) {
+            if (tries >= kLinkTries) {
+                set_status(d.ctl, SVDAG_ERR_TIMEOUT);
+                break;
+            }
+            __nanosleep(64);
+            next = *reinterpret_cast<volatile uint32_t*>(link);
+        }
+        if (next == kLinking || next == kEnd) // timed out, or the allocation failed (and latched its error)
+            next = kNone;
+    }
+    return g.bcast(next, 0);
 }
 
 constexpr uint32_t kMaxChain = 1u << 14; // bound on chain walks (16K slabs in one bucket only happens on a corrupt chain)
@@ -664,7 +669,7 @@ __device__ __forceinline__ uint32_t table_find(const Grp<G>& g, const DevDag& d,
             if (item_equals<G, LD_DEFAULT>(g, handle_ptr(d, item), key))
                 return item;
         }
-        if (next == kEnd)
+        if (next == kEnd || next == kLinking)
             return kNone;
         if (!slab_ok(d, next)) {
             set_status(d.ctl, SVDAG_ERR_CORRUPT);
@@ -719,7 +724,7 @@ __device__ __forceinline__ uint32_t claim_in_slab(const Grp<G>& g, const DevDag&
 // Unconditional insert (CompactAccelerationHashTable::addAsWarp, compact_acceleration_hash_table.h:63-121):
 // the key gets a fresh slot even when an equal key is stored already.
 template <int G>
-__device__ __forceinline__ uint32_t table_add(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key, Spare& spare)
+__device__ __forceinline__ uint32_t table_add(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key)
 {
     const uint32_t cls = key.n - 2u;
     if (key.n < 2u || key.n > 10u || t.numBuckets[cls] == 0) {
@@ -737,17 +742,10 @@ __device__ __forceinline__ uint32_t table_add(const Grp<G>& g, const DevDag& d, 
             write_item<G>(g, handle_ptr(d, item), key);
             return item;
         }
-        if (next == kEnd) {
-            take_spare<G>(g, d, t, spare, key.n);
-            if (spare.slab == kNone)
+        if (next == kEnd || next == kLinking) {
+            next = append_slab<G>(g, d, t, slab, key.n);
+            if (next == kNone)
                 return kNone;
-            uint32_t linked = kNone;
-            if (g.lane == 0)
-                linked = link_slab(d, slab, spare.slab);
-            linked = g.bcast(linked, 0);
-            if (linked == spare.slab)
-                spare.slab = kNone;
-            next = linked;
         }
         if (!slab_ok(d, next)) {
             set_status(d.ctl, SVDAG_ERR_CORRUPT);
@@ -766,7 +764,7 @@ constexpr uint32_t kLockTries = 1u << 20; // bound on waiting for a bucket lock 
 // final tag published, so concurrent probes of other keys never compare a half-written item.
 template <int G>
 __device__ __forceinline__ uint32_t table_find_or_insert_one(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key,
-    Spare& spare, bool& inserted);
+    bool& inserted);
 
 // Insert modes of table_find_or_insert: the default (keys that no other group of the launch looks
 // up) and shared (several threads may insert the same key at once: under the bucket lock).
@@ -779,7 +777,7 @@ enum : int { kInsertLaunch = 0, kInsertShared = 1 };
 // another; the wait for a lock is bounded and ends with SVDAG_ERR_TIMEOUT.
 template <int G, int MODE = kInsertLaunch>
 __device__ __forceinline__ uint32_t table_find_or_insert(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key,
-    Spare& spare, bool& inserted)
+    bool& inserted)
 {
     if constexpr (MODE == kInsertShared && G == 1) {
         inserted = false;
@@ -798,18 +796,18 @@ __device__ __forceinline__ uint32_t table_find_or_insert(const Grp<G>& g, const 
             __nanosleep(32);
         }
         __threadfence(); // acquire: the previous holder's item and tag are visible
-        const uint32_t h = table_find_or_insert_one<G>(g, d, t, key, spare, inserted);
+        const uint32_t h = table_find_or_insert_one<G>(g, d, t, key, inserted);
         __threadfence(); // release: this holder's item and tag are visible before the lock is free
         atomicExch(lock, 0u);
         return h;
     } else {
-        return table_find_or_insert_one<G>(g, d, t, key, spare, inserted);
+        return table_find_or_insert_one<G>(g, d, t, key, inserted);
     }
 }
 
 template <int G>
 __device__ __forceinline__ uint32_t table_find_or_insert_one(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key,
-    Spare& spare, bool& inserted)
+    bool& inserted)
 {
     inserted = false;
     const uint32_t cls = key.n - 2u;
@@ -844,7 +842,7 @@ __device__ __forceinline__ uint32_t table_find_or_insert_one(const Grp<G>& g, co
             openEmpty = empty;
             openBody = body;
         }
-        if (next == kEnd)
+        if (next == kEnd || next == kLinking)
             break;
         if (!slab_ok(d, next)) {
             set_status(d.ctl, SVDAG_ERR_CORRUPT);
@@ -878,17 +876,10 @@ __device__ __forceinline__ uint32_t table_find_or_insert_one(const Grp<G>& g, co
         probe_header<G, true>(g, slab_ptr(d, slab), tag, next, body, empty, &snap);
         if (empty)
             continue; // a slot was freed up meanwhile (cannot happen during edits, kept for safety)
-        if (next == kEnd) {
-            take_spare<G>(g, d, t, spare, key.n);
-            if (spare.slab == kNone)
+        if (next == kEnd || next == kLinking) {
+            next = append_slab<G>(g, d, t, slab, key.n);
+            if (next == kNone)
                 return kNone;
-            uint32_t linked = kNone;
-            if (g.lane == 0)
-                linked = link_slab(d, slab, spare.slab);
-            linked = g.bcast(linked, 0);
-            if (linked == spare.slab)
-                spare.slab = kNone;
-            next = linked;
         }
         if (!slab_ok(d, next)) {
             set_status(d.ctl, SVDAG_ERR_CORRUPT);

@@ -914,7 +914,7 @@ __device__ void ph_dedup_level(const DevDag& d, uint32_t level, char* scratch)
 // handle, or kNone when the item came out empty.
 template <int MODE>
 __device__ uint32_t merge_single(const DevDag& d, uint32_t level, uint32_t* w, const uint32_t* repC, const uint32_t* hC,
-    const Grp<1>& g, Spare& spare, unsigned long long& added)
+    const Grp<1>& g, unsigned long long& added)
 {
     EditCounters& E = *d.edit;
     const uint32_t LL = d.leafLevel;
@@ -942,8 +942,7 @@ __device__ uint32_t merge_single(const DevDag& d, uint32_t level, uint32_t* w, c
         atomicAdd(&E.repPerClass[level][key.n - 2], 1u);
     const DevTable t = d.ctl->tables[level];
     bool ins = false;
-    const uint32_t h = table_find_or_insert<1, MODE>(g, d, t, key, spare, ins);
-    release_spare<1>(g, d, t, spare);
+    const uint32_t h = table_find_or_insert<1, MODE>(g, d, t, key, ins);
     added += ins ? 1u : 0u;
     return h;
 }
@@ -975,7 +974,6 @@ __device__ void ph_merge_level(const DevDag& d, uint32_t level, char* scratch)
     uint32_t* items = reinterpret_cast<uint32_t*>(scratch + E.offN[level]);
     const DevTable t = d.ctl->tables[level];
     Grp<1> g;
-    Spare spare;
     uint32_t full = 0, reps = 0, added = 0;
     for (uint32_t i = ph_block(d) * blockDim.x + threadIdx.x; i < n; i += ph_grid(d) * blockDim.x) {
         uint32_t* it = items + (size_t)i * kItemStride;
@@ -1007,10 +1005,9 @@ __device__ void ph_merge_level(const DevDag& d, uint32_t level, char* scratch)
         if (E.builder) // the scene builder sizes the level tables from these
             atomicAdd(&E.repPerClass[level][key.n - 2], 1u);
         bool ins = false;
-        handle[i] = table_find_or_insert<1, SHARED ? kInsertShared : kInsertLaunch>(g, d, t, key, spare, ins);
+        handle[i] = table_find_or_insert<1, SHARED ? kInsertShared : kInsertLaunch>(g, d, t, key, ins);
         added += ins ? 1u : 0u;
     }
-    release_spare<1>(g, d, t, spare);
     if (full)
         atomicAdd(&E.ffCount[level], full);
     if (reps)
@@ -1034,7 +1031,6 @@ __device__ void ph_insert_level(const DevDag& d, const DevTable& t, uint32_t lev
     const uint32_t* items = reinterpret_cast<const uint32_t*>(scratch + E.offN[level]);
     Grp<G> g;
     const uint32_t groupsPerBlock = blockDim.x / G;
-    Spare spare;
     uint32_t added = 0;
     for (uint32_t i = ph_block(d) * groupsPerBlock + threadIdx.x / G; i < n; i += ph_grid(d) * groupsPerBlock) {
         if (rep[i] != i)
@@ -1042,13 +1038,12 @@ __device__ void ph_insert_level(const DevDag& d, const DevTable& t, uint32_t lev
         Key<G> key;
         load_key<G>(g, items + (size_t)i * kItemStride, kItemStride, t.kind, key);
         bool ins = false;
-        const uint32_t h = table_find_or_insert<G>(g, d, t, key, spare, ins);
+        const uint32_t h = table_find_or_insert<G>(g, d, t, key, ins);
         if (g.lane == 0) {
             handle[i] = h;
             added += ins ? 1u : 0u;
         }
     }
-    release_spare<G>(g, d, t, spare);
     if (added)
         atomicAdd(&E.added, (unsigned long long)added);
 }
@@ -1333,7 +1328,6 @@ __global__ void __launch_bounds__(1024) k_edit_spines(DevDag d, const DevEditor*
     DevDag dk = d;
     dk.solo = 1;
     Grp<1> g;
-    Spare spare;
     unsigned long long added = 0;
     for (int li = (int)maxTop - 1; li >= 0; --li) {
         const uint32_t l = (uint32_t)li;
@@ -1375,7 +1369,7 @@ __global__ void __launch_bounds__(1024) k_edit_spines(DevDag d, const DevEditor*
             w[0] = mask | (1u << (13 + ck));
             const uint32_t childHandle = ver[l + 1][k];
             const uint32_t regRep[1] = { childHandle == kNone ? kEmptyRep : 0u }, regHandle[1] = { childHandle };
-            const uint32_t hn = merge_single<kInsertShared>(dk, l, w, regRep, regHandle, g, spare, added);
+            const uint32_t hn = merge_single<kInsertShared>(dk, l, w, regRep, regHandle, g, added);
             if (hn == kNone && (w[0] & 0xFFu) != 0) // not emptied: the insert failed
                 atomicMin(&failAt, k);
             ver[l][k] = hn;

@@ -90,7 +90,6 @@ __global__ void k_insert_canonical(DevDag d, DevTable t, uint32_t level)
     if (threadIdx.x != 0 || blockIdx.x != 0)
         return;
     Grp<1> g;
-    Spare spare;
     for (uint32_t m = 0; m < SVDAG_NUM_MATERIALS; ++m) {
         Key<1> key;
         if (level == d.leafLevel) { // fully filled leaf of material m (my_gpu_hash_dag.cu:40-49)
@@ -107,9 +106,8 @@ __global__ void k_insert_canonical(DevDag d, DevTable t, uint32_t level)
         }
         hash_words(key.w, key.n, key.ha, key.hb);
         bool inserted;
-        d.ctl->fullyFilled[level][m] = table_find_or_insert<1>(g, d, t, key, spare, inserted);
+        d.ctl->fullyFilled[level][m] = table_find_or_insert<1>(g, d, t, key, inserted);
     }
-    release_spare<1>(g, d, t, spare);
 }
 
 svdag_status insert_canonical(svdag_ctx* ctx, uint32_t level, cudaStream_t s)
@@ -173,7 +171,6 @@ __global__ void __launch_bounds__(256) k_table_op(DevDag d, DevTable t, const ui
     Grp<G> g;
     const uint32_t groupsPerBlock = blockDim.x / G;
     const unsigned long long stride = (unsigned long long)gridDim.x * groupsPerBlock;
-    Spare spare;
     for (unsigned long long i = blockIdx.x * groupsPerBlock + threadIdx.x / G; i < n; i += stride) {
         if (reps && reps[i] != i)
             continue;
@@ -190,15 +187,14 @@ __global__ void __launch_bounds__(256) k_table_op(DevDag d, DevTable t, const ui
         if constexpr (OP == OP_FIND) {
             h = table_find<G>(g, d, t, key);
         } else if constexpr (OP == OP_ADD) {
-            h = table_add<G>(g, d, t, key, spare);
+            h = table_add<G>(g, d, t, key);
         } else {
             bool ins;
-            h = table_find_or_insert<G>(g, d, t, key, spare, ins);
+            h = table_find_or_insert<G>(g, d, t, key, ins);
         }
         if (g.lane == 0)
             out[i] = h;
     }
-    release_spare<G>(g, d, t, spare);
 }
 
 // Batch dedup into an open-addressing scratch table of 64-bit entries (tag hash << 32 | index+1).
