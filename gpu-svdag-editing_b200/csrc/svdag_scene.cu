@@ -390,7 +390,7 @@ svdag_status run_scene_build(svdag_ctx* ctx, const svdag_terrain_params* p, cuda
         unsigned long long per[kNumClasses];
         SVDAG_TRY(table_class_counts(ctx, ctx->levelTables[level], per, counters, s));
         for (uint32_t c = 0; c < kNumClasses; ++c)
-            buckets[level][c] = (uint32_t)std::max<unsigned long long>(1, (per[c] + ctx->loadFactor - 1) / ctx->loadFactor);
+            buckets[level][c] = (uint32_t)std::max<unsigned long long>(min_level_buckets(ctx), (per[c] + ctx->loadFactor - 1) / ctx->loadFactor);
     }
     // Final pass into exactly sized tables.
     SVDAG_TRY(reset_dag(ctx, s));

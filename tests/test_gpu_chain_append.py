@@ -34,3 +34,19 @@ def test_one_bucket_chain_has_no_spare_slabs(svdag_lib, lanes, n):
     dag.sync()
     assert np.array_equal(got.cpu().numpy().view(np.uint32)[:, :3], words)
     dag.free()
+
+
+def test_a_level_table_starts_with_room_for_versions(svdag_lib):
+    """The root of a scene is one item, but each edit adds a version of it: 60 edits fit the first
+    slabs of the root's table, with no chain."""
+    import svdag.workloads as w
+
+    dag = svdag_lib.MyGPUHashDAG(10, pool_bytes=2 << 30)
+    dag.build_terrain(**w.C0_TERRAIN)
+    for tool, material, center, radius in w.c0_edits(60):
+        dag.edit(w.make_edit(tool, material, center, min(radius, 12.0)))
+    dag.sync()
+    st = dag.table(0).stats()
+    assert st.items > 30
+    assert st.overflow_slabs == 0
+    dag.free()
