@@ -79,6 +79,7 @@ struct EditCounters {
     unsigned long long offW[kMaxLevels]; // scratch byte offset of each level's work items
     unsigned long long offN[kMaxLevels]; // scratch byte offset of each level's SVO items
     unsigned long long buildTop; // end of the top-down allocations
+    unsigned long long offM[kMaxLevels]; // scratch byte offset of each level's merge arrays (merge_layout_at)
     uint32_t rootBefore, rootAfter;
     uint32_t overflow; // scratch arena exhausted
     uint32_t builder; // scene build: merge even without leaves, discovery on every level

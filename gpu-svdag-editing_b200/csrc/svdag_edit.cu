@@ -441,29 +441,32 @@ __device__ void ph_build_leaves(const DevDag& d, const DevEditor& e, char* scrat
     if (E.overflow || (n == 0 && !E.builder))
         return;
     // Reserve and clear the dedup tables of every level for the bottom-up phase.
-    // The dedup tables of all levels form one contiguous run per level; walk the layout once (from
-    // the leaf level up, the order merge_layout assigns) instead of recomputing it per level.
+    // The dedup tables of all levels form one contiguous run per level, from the leaf level up.
     const uint32_t* cnt = E.count; // final: the top-down phases are done
-    const MergeLayout top = merge_layout(cnt, buildTop, 0, LL);
-    if (top.end > scratchBytes) {
-        if (threadIdx.x == 0)
-            atomicExch(&E.overflow, 1u);
-        return;
+    {
+        const bool first = ph_block(d) == 0 && threadIdx.x == 0;
+        unsigned long long off = buildTop;
+        for (int l = (int)LL; l >= 0; --l) {
+            if (first)
+                E.offM[l] = off;
+            off = merge_layout_at(off, cnt[l]).end;
+        }
+        if (off > scratchBytes) {
+            if (threadIdx.x == 0)
+                atomicExch(&E.overflow, 1u);
+            return;
+        }
     }
     const unsigned long long tid = ph_block(d) * (unsigned long long)blockDim.x + threadIdx.x;
     const unsigned long long nthreads = (unsigned long long)ph_grid(d) * blockDim.x;
     {
         unsigned long long off = buildTop;
         for (int l = (int)LL; l >= 0; --l) {
-            const unsigned long long nl = cnt[l];
-            uint32_t cap = 2;
-            while (cap < 2ull * nl)
-                cap <<= 1;
-            const unsigned long long table = align256(align256(off + 4 * nl) + 4 * nl);
-            uint4* t = reinterpret_cast<uint4*>(scratch + table);
-            for (unsigned long long j = tid; j < cap / 2; j += nthreads)
+            const MergeLayout m = merge_layout_at(off, cnt[l]);
+            uint4* t = reinterpret_cast<uint4*>(scratch + m.table);
+            for (unsigned long long j = tid; j < m.cap / 2; j += nthreads)
                 t[j] = make_uint4(0, 0, 0, 0);
-            off = align256(table + 8ull * cap);
+            off = m.end;
         }
     }
 
@@ -700,17 +703,6 @@ __device__ __forceinline__ bool discovery_gate(const EditCounters& E, uint32_t l
     return ranBelow && E.ffCount[level + 1] > 0;
 }
 
-// Value of slot j (0..7) of a register array without dynamic indexing (which would put the array in
-// local memory).
-__device__ __forceinline__ uint32_t sel8(const uint32_t (&v)[8], uint32_t j)
-{
-    uint32_t r = v[0];
-#pragma unroll
-    for (uint32_t k = 1; k < 8; ++k)
-        r = j == k ? v[k] : r;
-    return r;
-}
-
 // updateChildPointers + discover_fully_filled for one node held in registers
 // (my_gpu_hash_dag_edits.cu:44-150). Returns true when the node was found fully filled. Every slot is
 // handled with static indices and the loads of all children are issued together, stage by stage.
@@ -758,10 +750,16 @@ __device__ __forceinline__ bool fix_node(const DevDag& d, uint32_t level, bool g
             keep |= 1u << j;
         }
     uint32_t outW[8];
+    // slot j moves to the place its rank among the kept slots gives it (a rank is at most the slot)
 #pragma unroll
-    for (uint32_t p = 0; p < 8; ++p) {
-        const uint32_t j = (uint32_t)__fns(keep, 0, (int)p + 1);
-        outW[p] = j < 8 ? sel8(h, j) : 0u;
+    for (uint32_t p = 0; p < 8; ++p)
+        outW[p] = 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) {
+        const uint32_t rank = (keep >> j) & 1u ? (uint32_t)__popc(keep & ((1u << j) - 1u)) : 8u;
+#pragma unroll
+        for (uint32_t p = 0; p <= j; ++p)
+            outW[p] = rank == p ? h[j] : outW[p];
     }
     uint32_t header = newMask;
     bool full = false;
@@ -851,7 +849,7 @@ __device__ void ph_fix_level(const DevDag& d, uint32_t level, uint32_t builder, 
     const bool gate = discovery_gate(E, level, LL, builder);
     if (ph_block(d) == 0 && threadIdx.x == 0)
         E.ffRan[level] = gate ? 1u : 0u;
-    const MergeLayout ch = merge_layout(E.count, E.buildTop, level + 1, LL);
+    const MergeLayout ch = merge_layout_at(E.offM[level + 1], E.count[level + 1]);
     const uint32_t* repC = reinterpret_cast<const uint32_t*>(scratch + ch.rep);
     const uint32_t* hC = reinterpret_cast<const uint32_t*>(scratch + ch.handle);
     uint32_t* nodes = reinterpret_cast<uint32_t*>(scratch + E.offN[level]);
@@ -881,7 +879,7 @@ __device__ void ph_dedup_level(const DevDag& d, uint32_t level, char* scratch)
         return;
     const uint32_t LL = d.leafLevel;
     const uint32_t n = E.count[level];
-    const MergeLayout m = merge_layout(E.count, E.buildTop, level, LL);
+    const MergeLayout m = merge_layout_at(E.offM[level], n);
     uint32_t* rep = reinterpret_cast<uint32_t*>(scratch + m.rep);
     unsigned long long* table = reinterpret_cast<unsigned long long*>(scratch + m.table);
     const uint32_t* items = reinterpret_cast<const uint32_t*>(scratch + E.offN[level]);
@@ -964,8 +962,8 @@ __device__ void ph_merge_level(const DevDag& d, uint32_t level, char* scratch)
     const bool gate = isLeaf ? false : discovery_gate(E, level, LL, E.builder);
     if (!isLeaf && ph_block(d) == 0 && threadIdx.x == 0)
         E.ffRan[level] = gate ? 1u : 0u;
-    const MergeLayout m = merge_layout(E.count, E.buildTop, level, LL);
-    const MergeLayout ch = isLeaf ? m : merge_layout(E.count, E.buildTop, level + 1, LL);
+    const MergeLayout m = merge_layout_at(E.offM[level], n);
+    const MergeLayout ch = isLeaf ? m : merge_layout_at(E.offM[level + 1], E.count[level + 1]);
     const uint32_t* repC = reinterpret_cast<const uint32_t*>(scratch + ch.rep);
     const uint32_t* hC = reinterpret_cast<const uint32_t*>(scratch + ch.handle);
     uint32_t* rep = reinterpret_cast<uint32_t*>(scratch + m.rep);
@@ -1025,7 +1023,7 @@ __device__ void ph_insert_level(const DevDag& d, const DevTable& t, uint32_t lev
     if (!merge_live(d))
         return;
     const uint32_t n = E.count[level];
-    const MergeLayout m = merge_layout(E.count, E.buildTop, level, d.leafLevel);
+    const MergeLayout m = merge_layout_at(E.offM[level], n);
     const uint32_t* rep = reinterpret_cast<const uint32_t*>(scratch + m.rep);
     uint32_t* handle = reinterpret_cast<uint32_t*>(scratch + m.handle);
     const uint32_t* items = reinterpret_cast<const uint32_t*>(scratch + E.offN[level]);
@@ -1060,7 +1058,7 @@ __device__ void ph_edit_end(const DevDag& d, char* scratch, uint32_t builder, ui
         if (!d.solo) // a subtree edit's overflow is reported by k_edit_spines, for that edit alone
             set_status(c, SVDAG_ERR_OOM);
     } else if ((E.count[d.leafLevel] != 0 || builder) && E.err == 0) {
-        const MergeLayout m = merge_layout(E.count, E.buildTop, E.startLevel, d.leafLevel);
+        const MergeLayout m = merge_layout_at(E.offM[E.startLevel], E.count[E.startLevel]);
         const uint32_t r = reinterpret_cast<const uint32_t*>(scratch + m.rep)[0];
         const uint32_t h = r == kEmptyRep ? kNone : reinterpret_cast<const uint32_t*>(scratch + m.handle)[r];
         if (tileOut)

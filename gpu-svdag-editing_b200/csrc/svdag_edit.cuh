@@ -75,34 +75,39 @@ struct MergeLayout {
     uint32_t cap;
 };
 
-// Scratch layout of the bottom-up phase; every thread recomputes it from the final level counts
-// (count has kMaxLevels entries). The counts are all loaded before the walk over the levels, and the
-// walk is unrolled, so the counts stay in registers and cost one round trip.
+// Entries of the dedup table of n items: the smallest power of two of at least 2n (and 2).
+__host__ __device__ inline uint32_t dedup_cap(uint32_t n)
+{
+    if (n <= 1)
+        return 2;
+#ifdef __CUDA_ARCH__
+    return 1u << (32 - __clz(2u * n - 1u));
+#else
+    return 1u << (32 - __builtin_clz(2u * n - 1u));
+#endif
+}
+
+// The merge arrays of a level of n items that starts at scratch byte `off`.
+__host__ __device__ inline MergeLayout merge_layout_at(unsigned long long off, uint32_t n)
+{
+    MergeLayout m {};
+    m.cap = dedup_cap(n);
+    m.rep = off;
+    m.handle = align256(m.rep + 4ull * n);
+    m.table = align256(m.handle + 4ull * n);
+    m.end = align256(m.table + 8ull * m.cap);
+    return m;
+}
+
+// Scratch layout of the bottom-up phase: the levels from the leaves up, one after another. The leaf
+// phase walks it once and stores each level's start (EditCounters::offM) for the merge phases: walking
+// it in every thread of every merge launch, with the capacity found by a doubling loop, was about
+// 3 us of each launch.
 __host__ __device__ inline MergeLayout merge_layout(const uint32_t* count, unsigned long long buildTop, uint32_t level, uint32_t leafLevel)
 {
-    uint32_t c[kMaxLevels];
-#pragma unroll
-    for (uint32_t l = 0; l < kMaxLevels; ++l)
-        c[l] = count[l];
-    unsigned long long off = buildTop;
-    MergeLayout m {};
-#pragma unroll
-    for (int l = (int)kMaxLevels - 1; l >= 0; --l) {
-        if (l > (int)leafLevel)
-            continue;
-        const unsigned long long n = c[l];
-        uint32_t cap = 2;
-        while (cap < 2ull * n)
-            cap <<= 1;
-        m.rep = off;
-        m.handle = align256(m.rep + 4 * n);
-        m.table = align256(m.handle + 4 * n);
-        m.end = align256(m.table + 8ull * cap);
-        m.cap = cap;
-        if ((uint32_t)l == level)
-            return m;
-        off = m.end;
-    }
+    MergeLayout m = merge_layout_at(buildTop, count[leafLevel]);
+    for (int l = (int)leafLevel - 1; l >= (int)level; --l)
+        m = merge_layout_at(m.end, count[l]);
     return m;
 }
 
