@@ -205,52 +205,56 @@ __device__ __forceinline__ uint32_t voxel_op(const DevEditor& e, const AxisTerm&
     return OP_SUBDIVIDE;
 }
 
-// MyGpuCopyEditor::should_edit with state (the "#if 1" form, my_gpu_dag_editors.h:173-217).
-__device__ uint32_t copy_should_edit(const DevEditor& e, const DevDag& d, uint32_t px, uint32_t py, uint32_t pz, uint32_t depth,
-    const CopyParent* in, CopyParent* out)
+// MyGpuCopyEditor::should_edit with state (the "#if 1" form, my_gpu_dag_editors.h:173-217): the children of
+// the source parents `in` that overlap the node's source box, as eight bits a parent. The overlap test
+// (aabbOverlap, :121-125) is per axis and a parent has two child halves an axis, so six comparisons of
+// pairs decide its eight children. 0 = no source child (or no overlap with the destination box): Keep.
+__device__ __forceinline__ unsigned long long copy_overlaps(const DevEditor& e, const DevDag& d, uint32_t px, uint32_t py, uint32_t pz,
+    uint32_t depth, const CopyParent* in)
 {
     const float nmin[3] = { float(px << depth), float(py << depth), float(pz << depth) };
     const float nodeSize = float(1u << depth);
     const float nmax[3] = { nmin[0] + nodeSize, nmin[1] + nodeSize, nmin[2] + nodeSize };
     if (!box_overlap(e, nmin, nmax))
-        return OP_KEEP;
+        return 0;
     float smin[3], smax[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         smin[a] = cmaxf(nmin[a], e.bmin[a]) + e.fDestToSource[a];
         smax[a] = cminf(smin[a] + nodeSize, e.bmax[a] + e.fDestToSource[a]);
     }
-    const uint32_t parentLevel = e.levels - depth - 1;
-    (void)parentLevel;
-    uint32_t numOut = 0;
+    auto meets = [&](int a, uint32_t cell) {
+        const float lo = float(cell << depth), hi = lo + nodeSize;
+        return !(lo >= smax[a] || hi <= smin[a] || smin[a] >= hi || smax[a] <= lo);
+    };
+    unsigned long long out = 0;
+#pragma unroll
     for (uint32_t p = 0; p < 8; ++p) {
         const CopyParent par = in[p];
         if (par.handle == kNone)
             break;
-        const uint32_t* node = item_ptr(d, par.handle);
-        const uint32_t mask = node[0] & 0xFFu;
-        for (uint32_t c = 0; c < 8; ++c) {
-            if (!(mask & (1u << c)))
-                continue;
-            const uint32_t cx = (par.x << 1) | ((c >> 2) & 1u), cy = (par.y << 1) | ((c >> 1) & 1u), cz = (par.z << 1) | (c & 1u);
-            const float cmn[3] = { float(cx << depth), float(cy << depth), float(cz << depth) };
-            const float cmx[3] = { cmn[0] + nodeSize, cmn[1] + nodeSize, cmn[2] + nodeSize };
-            // aabbOverlap, :121-125
-            const bool ov = !(cmn[0] >= smax[0] || cmn[1] >= smax[1] || cmn[2] >= smax[2] || cmx[0] <= smin[0] || cmx[1] <= smin[1]
-                || cmx[2] <= smin[2] || smin[0] >= cmx[0] || smin[1] >= cmx[1] || smin[2] >= cmx[2] || smax[0] <= cmn[0]
-                || smax[1] <= cmn[1] || smax[2] <= cmn[2]);
-            if (ov && numOut < 8) {
-                out[numOut].handle = node[1 + __popc(mask & ((1u << c) - 1u))];
-                out[numOut].x = cx;
-                out[numOut].y = cy;
-                out[numOut].z = cz;
-                ++numOut;
-            }
-        }
+        uint32_t m = item_ptr(d, par.handle)[0] & 0xFFu;
+        m &= (meets(0, par.x << 1) ? 0x0Fu : 0u) | (meets(0, (par.x << 1) | 1u) ? 0xF0u : 0u);
+        m &= (meets(1, par.y << 1) ? 0x33u : 0u) | (meets(1, (par.y << 1) | 1u) ? 0xCCu : 0u);
+        m &= (meets(2, par.z << 1) ? 0x55u : 0u) | (meets(2, (par.z << 1) | 1u) ? 0xAAu : 0u);
+        out |= (unsigned long long)m << (8u * p);
     }
-    if (numOut != 8)
-        out[numOut].handle = kNone;
-    return numOut == 0 ? OP_KEEP : OP_SUBDIVIDE;
+    return out;
+}
+// Writes the source children that copy_overlaps found (at most eight; a shorter list ends with kNone).
+__device__ __forceinline__ void copy_emit(const DevDag& d, const CopyParent* in, unsigned long long found, CopyParent* out)
+{
+    uint32_t n = 0;
+    while (found && n < 8) {
+        const uint32_t bit = (uint32_t)__ffsll((long long)found) - 1u, c = bit & 7u;
+        found &= found - 1ull;
+        const CopyParent par = in[bit >> 3];
+        const uint32_t* node = item_ptr(d, par.handle);
+        out[n++] = CopyParent { (par.x << 1) | (c >> 2), (par.y << 1) | ((c >> 1) & 1u), (par.z << 1) | (c & 1u),
+            node[1 + __popc(node[0] & ((1u << c) - 1u))] };
+    }
+    if (n != 8)
+        out[n].handle = kNone;
 }
 
 // material of voxel `v` of the leaf at `leaf` (get_material, my_gpu_base_dag.h:293-316)
@@ -369,11 +373,12 @@ __device__ void ph_build_level(const DevDag& d, const DevEditor& e, uint32_t lev
         }
         const uint32_t cx = (w.x << 1) | ((c >> 2) & 1u), cy = (w.y << 1) | ((c >> 1) & 1u), cz = (w.z << 1) | (c & 1u);
         uint32_t op = OP_KEEP;
-        CopyParent childState[8];
+        unsigned long long sources = 0; // copy: the source children of the node
+        const CopyParent* parents = reinterpret_cast<const CopyParent*>(scratch + offW + i * stride + 16);
         if (active) {
             if constexpr (TOOL == SVDAG_TOOL_COPY) {
-                const CopyParent* in = reinterpret_cast<const CopyParent*>(scratch + offW + i * stride + 16);
-                op = copy_should_edit(e, d, cx, cy, cz, childDepth, in, childState);
+                sources = copy_overlaps(e, d, cx, cy, cz, childDepth, parents);
+                op = sources ? OP_SUBDIVIDE : OP_KEEP;
             } else {
                 op = should_edit<TOOL>(e, cx, cy, cz, childDepth, state, fillMat);
             }
@@ -392,11 +397,8 @@ __device__ void ph_build_level(const DevDag& d, const DevEditor& e, uint32_t lev
             const unsigned long long at = offWn + (unsigned long long)idx * stride;
             if (at + stride <= scratchBytes) {
                 *reinterpret_cast<WorkItem*>(scratch + at) = WorkItem { cx, cy, cz, child };
-                if constexpr (TOOL == SVDAG_TOOL_COPY) {
-                    CopyParent* out = reinterpret_cast<CopyParent*>(scratch + at + 16);
-                    for (int p = 0; p < 8; ++p)
-                        out[p] = childState[p];
-                }
+                if constexpr (TOOL == SVDAG_TOOL_COPY)
+                    copy_emit(d, parents, sources, reinterpret_cast<CopyParent*>(scratch + at + 16));
             } else {
                 atomicExch(&E.overflow, 1u);
             }
@@ -454,6 +456,7 @@ __device__ void ph_build_leaves(const DevDag& d, const DevEditor& e, char* scrat
 {
     __shared__ __align__(16) uint32_t packBuf[16][16]; // per warp of a block of up to 512 threads: 64 material bytes
     __shared__ uint2 erodeBuf[TOOL == SVDAG_TOOL_SPHERE_ERODE ? 16 : 1][27]; // erosion: per warp, the neighbour leaf masks
+    __shared__ __align__(16) uint32_t copyBuf[TOOL == SVDAG_TOOL_COPY ? 16 : 1][8][12]; // copy: per warp, the source leaves
     EditCounters& E = *d.edit;
     const uint32_t LL = d.leafLevel;
     const unsigned long long stride = work_stride(TOOL);
@@ -566,6 +569,43 @@ __device__ void ph_build_leaves(const DevDag& d, const DevEditor& e, char* scrat
                 nb[lane] = make_uint2(nlo, nhi);
             __syncwarp();
         }
+        // copy: a leaf's source box meets at most two leaves an axis; they are fetched once, all words at a
+        // time, into the slot of their place in that 2 x 2 x 2 block (absent ones read as empty)
+        uint32_t base[3] = {};
+        if constexpr (TOOL == SVDAG_TOOL_COPY) {
+            const uint32_t at[3] = { w.x << 2, w.y << 2, w.z << 2 };
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const int first = (int)at[a] + e.iDestToSource[a];
+                base[a] = (uint32_t)(first > 0 ? first : 0) >> 2;
+            }
+            CopyParent par { 0, 0, 0, kNone };
+            if (lane < 8)
+                par = reinterpret_cast<const CopyParent*>(scratch + offW + i * stride + 16)[lane];
+            const uint32_t ends = __ballot_sync(0xFFFFFFFFu, par.handle == kNone); // a list ends at its first kNone
+            const uint32_t rx = par.x - base[0], ry = par.y - base[1], rz = par.z - base[2];
+            uint32_t slot = (rx * 2u + ry) * 2u + rz;
+            if (lane + 1u >= (uint32_t)__ffs(ends) || rx > 1u || ry > 1u || rz > 1u)
+                slot = 8u;
+            uint32_t (*leaves)[12] = copyBuf[threadIdx.x >> 5];
+            __syncwarp();
+            if (lane < 8)
+                leaves[lane][0] = leaves[lane][1] = 0u;
+            __syncwarp();
+            uint32_t v[3], to[3];
+#pragma unroll
+            for (uint32_t r = 0; r < 3; ++r) {
+                const uint32_t k = lane + 32u * r, p = k / kItemStride;
+                const uint32_t hp = __shfl_sync(0xFFFFFFFFu, par.handle, p & 7u), sp = __shfl_sync(0xFFFFFFFFu, slot, p & 7u);
+                to[r] = p < 8u ? sp : 8u;
+                v[r] = to[r] < 8u ? item_ptr(d, hp)[k % kItemStride] : 0u;
+            }
+#pragma unroll
+            for (uint32_t r = 0; r < 3; ++r)
+                if (to[r] < 8u)
+                    leaves[to[r]][(lane + 32u * r) % kItemStride] = v[r];
+            __syncwarp();
+        }
         const uint32_t dx = ((lane >> 3) & 2u) | ((lane >> 2) & 1u), dy = ((lane >> 2) & 2u) | ((lane >> 1) & 1u), dz0 = lane & 1u;
         const uint32_t vx = (w.x << 2) | dx, vy = (w.y << 2) | dy, vz0 = (w.z << 2) | dz0;
         AxisTerm tx = {}, ty = {}, tz[2] = {};
@@ -660,24 +700,13 @@ __device__ void ph_build_leaves(const DevDag& d, const DevEditor& e, char* scrat
                         sy = sy > 0 ? sy : 0;
                         sz = sz > 0 ? sz : 0;
                         const uint32_t ux = (uint32_t)sx, uy = (uint32_t)sy, uz = (uint32_t)sz;
-                        const CopyParent* st = reinterpret_cast<const CopyParent*>(scratch + offW + i * stride + 16);
-                        uint32_t found = kNone;
-                        for (int p = 0; p < 8; ++p) {
-                            const CopyParent par = st[p];
-                            if (par.handle == kNone)
-                                break;
-                            if (par.x == (ux >> 2) && par.y == (uy >> 2) && par.z == (uz >> 2))
-                                found = par.handle;
-                        }
-                        if (found != kNone) {
-                            const uint32_t* src = item_ptr(d, found);
-                            const uint32_t bitIdx = ((ux & 1u) ? 4u : 0u) | ((uy & 1u) ? 2u : 0u) | ((uz & 1u) ? 1u : 0u) | ((ux & 2u) ? 32u : 0u)
-                                | ((uy & 2u) ? 16u : 0u) | ((uz & 2u) ? 8u : 0u);
-                            uint32_t m;
-                            if (leaf_get_material(src[0], src[1], src, bitIdx, m)) {
-                                out = true;
-                                mat = m;
-                            }
+                        const uint32_t* src = copyBuf[threadIdx.x >> 5][(((ux >> 2) - base[0]) * 2u + ((uy >> 2) - base[1])) * 2u + ((uz >> 2) - base[2])];
+                        const uint32_t bitIdx = ((ux & 1u) ? 4u : 0u) | ((uy & 1u) ? 2u : 0u) | ((uz & 1u) ? 1u : 0u) | ((ux & 2u) ? 32u : 0u)
+                            | ((uy & 2u) ? 16u : 0u) | ((uz & 2u) ? 8u : 0u);
+                        uint32_t m;
+                        if (leaf_get_material(src[0], src[1], src, bitIdx, m)) {
+                            out = true;
+                            mat = m;
                         }
                     } else { // removal tools
                         out = false;
