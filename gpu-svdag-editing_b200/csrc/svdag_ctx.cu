@@ -331,9 +331,7 @@ svdag_status svdag_create(const svdag_config* cfg, svdag_ctx** out)
     ctx->poolBytes = pool;
     ctx->ctl = reinterpret_cast<Control*>(ctx->pool);
     ctx->batch = ctx->pool + kCtlBytes;
-    ctx->batchBytes = kBatchBytes - 4096; // the last 4 KiB hold the editor queue of the phase launches
-    ctx->queue = reinterpret_cast<EditQueue*>(ctx->batch + ctx->batchBytes);
-    static_assert(sizeof(EditQueue) <= 4096, "editor queue too large");
+    ctx->batchBytes = kBatchBytes;
     ctx->scratch = ctx->pool + kCtlBytes + kBatchBytes;
     ctx->scratchBytes = scratch;
     // The rest: slab headers (a thirteenth: 32 bytes per slab, whose body of 24 items takes at least
@@ -377,9 +375,6 @@ svdag_status svdag_destroy(svdag_ctx* ctx)
     cudaSetDevice(ctx->device);
     for (auto* t : ctx->standalone)
         delete t;
-    for (auto& g : ctx->graphs)
-        if (g)
-            cudaGraphExecDestroy(g);
     cudaDeviceSynchronize();
     cudaFree(ctx->pool);
     delete ctx;

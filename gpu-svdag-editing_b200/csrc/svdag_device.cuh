@@ -758,59 +758,20 @@ __device__ __forceinline__ uint32_t table_add(const Grp<G>& g, const DevDag& d, 
     return kNone;
 }
 
-constexpr uint32_t kLockTries = 1u << 20; // bound on waiting for a bucket lock (about 30 ms)
-
-// Find-or-insert for keys that no other group of the same launch looks up (the DAG merge inserts
-// each distinct item once). A slot is claimed with the in-flight tag, the item written, then the
-// final tag published, so concurrent probes of other keys never compare a half-written item.
+// What a probe of a key's chain found when the key is not there: where an insert may start.
 template <int G>
-__device__ __forceinline__ uint32_t table_find_or_insert_one(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key,
-    bool& inserted);
+struct Probed {
+    uint32_t slab, body, empty; // the first slab of the chain with a free slot, else the tail
+    bool snapValid; // `snap` holds that slab's tag words
+    HdrSnap<G> snap;
+};
 
-// Insert modes of table_find_or_insert: the default (keys that no other group of the launch looks
-// up) and shared (several threads may insert the same key at once: under the bucket lock).
-enum : int { kInsertLaunch = 0, kInsertShared = 1 };
-
-// Find-or-insert. In the shared mode (one thread per key, G = 1), several threads may look up and
-// insert the same key at once (the blocks and the path threads of a group of subtree edits): the
-// lookup and insert then run under the bucket's lock (a striped lock word in d.locks), so the
-// second of two equal keys finds the first's published item. A holder only probes and inserts into its own chain, so no lock waits on
-// another; the wait for a lock is bounded and ends with SVDAG_ERR_TIMEOUT.
-template <int G, int MODE = kInsertLaunch>
-__device__ __forceinline__ uint32_t table_find_or_insert(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key,
-    bool& inserted)
-{
-    if constexpr (MODE == kInsertShared && G == 1) {
-        inserted = false;
-        const uint32_t cls = key.n - 2u;
-        if (key.n < 2u || key.n > 10u || t.numBuckets[cls] == 0 || !d.locks) {
-            set_status(d.ctl, SVDAG_ERR_INVALID);
-            return kNone;
-        }
-        uint32_t* lock = d.locks + (first_slab(t, cls, key.ha) & (kLockStripes - 1u));
-        uint32_t tries = 0;
-        while (atomicCAS(lock, 0u, 1u) != 0u) {
-            if (++tries >= kLockTries) {
-                set_status(d.ctl, SVDAG_ERR_TIMEOUT);
-                return kNone;
-            }
-            __nanosleep(32);
-        }
-        __threadfence(); // acquire: the previous holder's item and tag are visible
-        const uint32_t h = table_find_or_insert_one<G>(g, d, t, key, inserted);
-        __threadfence(); // release: this holder's item and tag are visible before the lock is free
-        atomicExch(lock, 0u);
-        return h;
-    } else {
-        return table_find_or_insert_one<G>(g, d, t, key, inserted);
-    }
-}
-
+// Looks a key up through L2 (other SMs' inserts of the same launch are seen). Returns the item, or kNone
+// and where to insert; `ok` is false when the lookup itself failed (its error is latched).
 template <int G>
-__device__ __forceinline__ uint32_t table_find_or_insert_one(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key,
-    bool& inserted)
+__device__ __forceinline__ uint32_t table_probe(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key, Probed<G>& at, bool& ok)
 {
-    inserted = false;
+    ok = false;
     const uint32_t cls = key.n - 2u;
     if (key.n < 2u || key.n > 10u || t.numBuckets[cls] == 0) {
         set_status(d.ctl, SVDAG_ERR_INVALID);
@@ -820,20 +781,21 @@ __device__ __forceinline__ uint32_t table_find_or_insert_one(const Grp<G>& g, co
     uint32_t slab = first_slab(t, cls, key.ha);
     uint32_t tail = slab, tailEmpty = 0, tailBody = 0;
     uint32_t open = kNone, openEmpty = 0, openBody = 0; // first slab of the chain with a free slot
-    HdrSnap<G> snap;
     for (uint32_t steps = 0;; ++steps) {
         if (steps >= kMaxChain) {
             set_status(d.ctl, SVDAG_ERR_CORRUPT);
             return kNone;
         }
         uint32_t next, body, empty;
-        uint32_t cand = probe_header<G, true>(g, slab_ptr(d, slab), tag, next, body, empty, &snap);
+        uint32_t cand = probe_header<G, true>(g, slab_ptr(d, slab), tag, next, body, empty, &at.snap);
         while (cand) {
             const uint32_t s = __ffs(cand) - 1u;
             cand &= cand - 1u;
             const uint32_t item = slot_handle(body, s, key.n);
-            if (item_equals<G, LD_L2>(g, handle_ptr(d, item), key))
+            if (item_equals<G, LD_L2>(g, handle_ptr(d, item), key)) {
+                ok = true;
                 return item;
+            }
         }
         tail = slab;
         tailEmpty = empty;
@@ -851,30 +813,60 @@ __device__ __forceinline__ uint32_t table_find_or_insert_one(const Grp<G>& g, co
         }
         slab = next;
     }
-    // Not present: claim a slot in the first slab that had one free (slots freed by garbage
-    // collection are reused before the chain grows), else at the tail of the chain.
+    // An insert claims a slot in the first slab that had one free (slots freed by garbage collection
+    // are reused before the chain grows), else at the tail of the chain.
     const bool atTail = open == kNone || open == tail;
-    slab = atTail ? tail : open;
-    uint32_t empty = atTail ? tailEmpty : openEmpty, body = atTail ? tailBody : openBody;
-    bool snapValid = atTail; // `snap` holds the tag words of the tail, the last slab probed
+    at.slab = atTail ? tail : open;
+    at.empty = atTail ? tailEmpty : openEmpty;
+    at.body = atTail ? tailBody : openBody;
+    at.snapValid = atTail; // `snap` holds the tag words of the tail, the last slab probed
+    ok = true;
+    return kNone;
+}
+
+// How an insert makes its item visible. kPublish: the slot is claimed with the in-flight tag, the item
+// written, then the final tag published, so that probes of other keys running at the same time never
+// compare a half-written item. kQuiet: nothing probes the table until the inserts are over (the caller
+// puts a barrier between lookups and inserts), so the slot is claimed with its final tag and nothing
+// waits for the item's stores. kSole: moreover no other thread inserts into the table, so the claim is
+// a plain store that nothing waits for either.
+enum : int { kPublish = 0, kQuiet = 1, kSole = 2 };
+
+template <int G, int HOW = kPublish>
+__device__ __forceinline__ uint32_t table_insert_probed(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key, Probed<G>& at)
+{
+    const uint32_t tag = tag_of(key.hb);
+    uint32_t slab = at.slab, empty = at.empty, body = at.body;
+    if constexpr (HOW == kSole && G == 1) {
+        if (empty && at.snapValid) {
+            const uint32_t start = (key.ha >> 8) % kSlots, up = empty >> start;
+            const uint32_t s = up ? start + (uint32_t)__ffs(up) - 1u : (uint32_t)__ffs(empty) - 1u;
+            slab_ptr(d, slab)[s >> 2] = at.snap.get(s >> 2, 0) | (tag << (8u * (s & 3u)));
+            const uint32_t item = slot_handle(body, s, key.n);
+            write_item<G>(g, handle_ptr(d, item), key);
+            return item;
+        }
+    }
+    bool snapValid = at.snapValid;
     for (uint32_t steps = 0; steps < kMaxChain; ++steps) {
         uint32_t s = 0;
-        const uint32_t item = claim_in_slab<G>(g, d, slab, body, empty, tag, key.n, true, s, key.ha >> 8, snapValid ? &snap : nullptr);
+        const uint32_t item = claim_in_slab<G>(g, d, slab, body, empty, tag, key.n, HOW == kPublish, s, key.ha >> 8, snapValid ? &at.snap : nullptr);
         snapValid = true;
         if (item != kNone) {
             write_item<G>(g, handle_ptr(d, item), key);
-            if constexpr (G == 1)
-                fence_release(); // the writer publishes: a release orders its item before the tag
-            else
-                __threadfence();
-            g.sync();
-            if (g.lane == 0)
-                atomicXor(slab_ptr(d, slab) + (s >> 2), (kTagBusy ^ tag) << (8u * (s & 3u)));
-            inserted = true;
+            if constexpr (HOW == kPublish) {
+                if constexpr (G == 1)
+                    fence_release(); // the writer publishes: a release orders its item before the tag
+                else
+                    __threadfence();
+                g.sync();
+                if (g.lane == 0)
+                    atomicXor(slab_ptr(d, slab) + (s >> 2), (kTagBusy ^ tag) << (8u * (s & 3u)));
+            }
             return item;
         }
         uint32_t next;
-        probe_header<G, true>(g, slab_ptr(d, slab), tag, next, body, empty, &snap);
+        probe_header<G, true>(g, slab_ptr(d, slab), tag, next, body, empty, &at.snap);
         if (empty)
             continue; // a slot was freed up meanwhile (cannot happen during edits, kept for safety)
         if (next == kEnd || next == kLinking) {
@@ -887,10 +879,61 @@ __device__ __forceinline__ uint32_t table_find_or_insert_one(const Grp<G>& g, co
             return kNone;
         }
         slab = next;
-        probe_header<G, true>(g, slab_ptr(d, slab), tag, next, body, empty, &snap);
+        probe_header<G, true>(g, slab_ptr(d, slab), tag, next, body, empty, &at.snap);
     }
     set_status(d.ctl, SVDAG_ERR_TIMEOUT);
     return kNone;
+}
+
+constexpr uint32_t kLockTries = 1u << 20; // bound on waiting for a bucket lock (about 30 ms)
+
+// Insert modes of table_find_or_insert: the default (keys that no other group of the launch looks
+// up) and shared (several threads may insert the same key at once: under the bucket lock).
+enum : int { kInsertLaunch = 0, kInsertShared = 1 };
+
+// Find-or-insert. In the shared mode (one thread per key, G = 1), several threads may look up and
+// insert the same key at once (the blocks and the path threads of a group of subtree edits). A key that
+// is there already is found without the lock (items are published after their words); a missing one is
+// looked up again and inserted under the bucket's lock (a striped lock word in d.locks), so the second of
+// two equal keys finds the first's published item. A holder only probes and inserts into its own chain,
+// so no lock waits on another; the wait for a lock is bounded and ends with SVDAG_ERR_TIMEOUT.
+template <int G, int MODE = kInsertLaunch>
+__device__ __forceinline__ uint32_t table_find_or_insert(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key, bool& inserted)
+{
+    inserted = false;
+    Probed<G> at;
+    bool ok;
+    uint32_t h = table_probe<G>(g, d, t, key, at, ok);
+    if (h != kNone || !ok)
+        return h;
+    if constexpr (MODE == kInsertShared && G == 1) {
+        if (!d.locks) {
+            set_status(d.ctl, SVDAG_ERR_INVALID);
+            return kNone;
+        }
+        uint32_t* lock = d.locks + (first_slab(t, key.n - 2u, key.ha) & (kLockStripes - 1u));
+        uint32_t tries = 0;
+        while (atomicCAS(lock, 0u, 1u) != 0u) {
+            if (++tries >= kLockTries) {
+                set_status(d.ctl, SVDAG_ERR_TIMEOUT);
+                return kNone;
+            }
+            __nanosleep(32);
+        }
+        __threadfence(); // acquire: the previous holder's item and tag are visible
+        h = table_probe<G>(g, d, t, key, at, ok);
+        if (h == kNone && ok) {
+            h = table_insert_probed<G>(g, d, t, key, at);
+            inserted = h != kNone;
+        }
+        __threadfence(); // release: this holder's item and tag are visible before the lock is free
+        atomicExch(lock, 0u);
+        return h;
+    } else {
+        h = table_insert_probed<G>(g, d, t, key, at);
+        inserted = h != kNone;
+        return h;
+    }
 }
 
 } // namespace svdag

@@ -802,42 +802,64 @@ __device__ __forceinline__ bool discovery_gate(const EditCounters& E, uint32_t l
     return ranBelow && E.ffCount[level + 1] > 0;
 }
 
+// The handles of the children built in this edit, from their level's arrays: their representative and,
+// loaded beside it, the handle stored under the child's own index, which is the answer when the child
+// is its own representative (only a duplicate needs the second, dependent load).
+struct ArrayChildren {
+    const uint32_t* rep;
+    const uint32_t* handle;
+    __device__ __forceinline__ void resolve(uint32_t built, uint32_t (&h)[8]) const
+    {
+        uint32_t r[8], own[8];
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            r[j] = (built >> j) & 1u ? rep[h[j]] : kEmptyRep;
+            own[j] = (built >> j) & 1u ? handle[h[j]] : kNone;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j)
+            if ((built >> j) & 1u)
+                h[j] = r[j] == kEmptyRep ? kNone : (r[j] == h[j] ? own[j] : handle[r[j]]);
+    }
+};
+// The same from resolved handles (kNone for an emptied child).
+struct ResolvedChildren {
+    const uint32_t* handle;
+    __device__ __forceinline__ void resolve(uint32_t built, uint32_t (&h)[8]) const
+    {
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j)
+            if ((built >> j) & 1u)
+                h[j] = handle[h[j]];
+    }
+};
+
 // updateChildPointers + discover_fully_filled for one node held in registers
 // (my_gpu_hash_dag_edits.cu:44-150). Returns true when the node was found fully filled. Every slot is
 // handled with static indices and the loads of all children are issued together, stage by stage.
-__device__ __forceinline__ bool fix_node(const DevDag& d, uint32_t level, bool gate, const uint32_t* repC, const uint32_t* hC,
-    uint32_t* w)
+template <class Children>
+__device__ __forceinline__ bool fix_node(const DevDag& d, uint32_t level, bool gate, const Children& children, uint32_t* w)
 {
     const uint32_t LL = d.leafLevel;
     const uint32_t mask = w[0] & 0xFFu;
     const uint32_t interm = w[0] >> 13;
     const uint32_t n = __popc(mask);
-    uint32_t cbit[8], h[8];
+    uint32_t cbit[8], h[8], built = 0;
     uint32_t rem = mask;
 #pragma unroll
     for (uint32_t j = 0; j < 8; ++j) {
         cbit[j] = rem ? (uint32_t)__ffs(rem) - 1u : 0u;
         rem &= rem - 1u;
         h[j] = w[1 + j];
+        built |= j < n && ((interm >> cbit[j]) & 1u) ? 1u << j : 0u;
     }
-    // Children built in this edit: their representative and, loaded beside it, the handle stored
-    // under the child's own index, which is the answer when the child is its own representative
-    // (only a duplicate needs the second, dependent load of its representative's handle).
-    uint32_t r[8], own[8];
-#pragma unroll
-    for (uint32_t j = 0; j < 8; ++j) {
-        const bool built = j < n && ((interm >> cbit[j]) & 1u);
-        r[j] = built ? repC[h[j]] : kEmptyRep;
-        own[j] = built ? hC[h[j]] : kNone;
-    }
+    children.resolve(built, h);
     const uint32_t* ff = d.ctl->fullyFilled[level + 1];
 #pragma unroll
     for (uint32_t j = 0; j < 8; ++j) {
         if (j >= n)
             h[j] = kNone;
-        else if ((interm >> cbit[j]) & 1u)
-            h[j] = r[j] == kEmptyRep ? kNone : (r[j] == h[j] ? own[j] : hC[r[j]]);
-        else if (h[j] >= kFillMarker && h[j] != kNone)
+        else if (!((built >> j) & 1u) && h[j] >= kFillMarker && h[j] != kNone)
             h[j] = ff[h[j] & 0xFu];
     }
     // Drop emptied children, keep the others in child order.
@@ -959,7 +981,7 @@ __device__ void ph_fix_level(const DevDag& d, uint32_t level, uint32_t builder, 
 #pragma unroll
         for (uint32_t j = 0; j < kItemStride; ++j)
             w[j] = node[j];
-        full += fix_node(d, level, gate, repC, hC, w) ? 1u : 0u;
+        full += fix_node(d, level, gate, ArrayChildren { repC, hC }, w) ? 1u : 0u;
 #pragma unroll
         for (uint32_t j = 0; j < kItemStride; ++j)
             node[j] = w[j];
@@ -1006,12 +1028,12 @@ __device__ void ph_dedup_level(const DevDag& d, uint32_t level, char* scratch)
 }
 
 // The bottom-up step of one SVO item held in w (one thread; the item is alone on its level, so it has
-// no duplicates): gated fully-filled discovery and child fix-up (children built in this edit are
-// looked up in repC / hC), then find-or-insert in the level table. Leaves w fixed; returns the item's
-// handle, or kNone when the item came out empty.
+// no duplicates): gated fully-filled discovery and child fix-up (`childHandle`: resolved handles of the
+// children built in this edit), then find-or-insert in the level table. Leaves w fixed; returns the
+// item's handle, or kNone when the item came out empty.
 template <int MODE>
-__device__ uint32_t merge_single(const DevDag& d, uint32_t level, uint32_t* w, const uint32_t* repC, const uint32_t* hC,
-    const Grp<1>& g, unsigned long long& added)
+__device__ uint32_t merge_single(const DevDag& d, uint32_t level, uint32_t* w, const uint32_t* childHandle, const Grp<1>& g,
+    unsigned long long& added)
 {
     EditCounters& E = *d.edit;
     const uint32_t LL = d.leafLevel;
@@ -1023,7 +1045,7 @@ __device__ uint32_t merge_single(const DevDag& d, uint32_t level, uint32_t* w, c
     if (!isLeaf) {
         const bool gate = discovery_gate(E, level, LL, E.builder);
         E.ffRan[level] = gate ? 1u : 0u;
-        if (fix_node(d, level, gate, repC, hC, key.w))
+        if (fix_node(d, level, gate, ResolvedChildren { childHandle }, key.w))
             E.ffCount[level] = 1;
 #pragma unroll
         for (uint32_t j = 0; j < kItemStride; ++j)
@@ -1035,9 +1057,7 @@ __device__ uint32_t merge_single(const DevDag& d, uint32_t level, uint32_t* w, c
     key.n = isLeaf ? dev_leaf_words(key.w[0], key.w[1]) : dev_node_words(key.w[0]);
     hash_words(key.w, key.n, key.ha, key.hb);
     E.repCount[level] = 1;
-    if (E.builder)
-        atomicAdd(&E.repPerClass[level][key.n - 2], 1u);
-    const DevTable t = d.ctl->tables[level];
+    const DevTable& t = d.ctl->tables[level];
     bool ins = false;
     const uint32_t h = table_find_or_insert<1, MODE>(g, d, t, key, ins);
     added += ins ? 1u : 0u;
@@ -1069,7 +1089,7 @@ __device__ void ph_merge_level(const DevDag& d, uint32_t level, char* scratch)
     uint32_t* handle = reinterpret_cast<uint32_t*>(scratch + m.handle);
     unsigned long long* table = reinterpret_cast<unsigned long long*>(scratch + m.table);
     uint32_t* items = reinterpret_cast<uint32_t*>(scratch + E.offN[level]);
-    const DevTable t = d.ctl->tables[level];
+    const DevTable& t = d.ctl->tables[level]; // in memory: a copy indexed by size class would live on the stack
     Grp<1> g;
     uint32_t full = 0, reps = 0, added = 0;
     for (uint32_t i = ph_block(d) * blockDim.x + threadIdx.x; i < n; i += ph_grid(d) * blockDim.x) {
@@ -1079,7 +1099,7 @@ __device__ void ph_merge_level(const DevDag& d, uint32_t level, char* scratch)
         for (uint32_t j = 0; j < kItemStride; ++j)
             key.w[j] = it[j];
         if (!isLeaf) {
-            full += fix_node(d, level, gate, repC, hC, key.w) ? 1u : 0u;
+            full += fix_node(d, level, gate, ArrayChildren { repC, hC }, key.w) ? 1u : 0u;
 #pragma unroll
             for (uint32_t j = 0; j < kItemStride; ++j)
                 it[j] = key.w[j];
@@ -1099,8 +1119,6 @@ __device__ void ph_merge_level(const DevDag& d, uint32_t level, char* scratch)
         if (r != i)
             continue;
         ++reps;
-        if (E.builder) // the scene builder sizes the level tables from these
-            atomicAdd(&E.repPerClass[level][key.n - 2], 1u);
         bool ins = false;
         handle[i] = table_find_or_insert<1, SHARED ? kInsertShared : kInsertLaunch>(g, d, t, key, ins);
         added += ins ? 1u : 0u;
@@ -1145,10 +1163,10 @@ __device__ void ph_insert_level(const DevDag& d, const DevTable& t, uint32_t lev
         atomicAdd(&E.added, (unsigned long long)added);
 }
 
-__device__ void ph_edit_end(const DevDag& d, char* scratch, uint32_t builder, uint32_t* tileOut, EditRecord* record)
+// Ends an edit: commits `root` (the handle the merges gave the edit's topmost node) when the edit reached
+// the leaves, and writes its record (one thread).
+__device__ void edit_end(const DevDag& d, uint32_t root, uint32_t builder, uint32_t* tileOut, EditRecord* record)
 {
-    if (threadIdx.x != 0 || ph_block(d) != 0)
-        return;
     Control* c = d.ctl;
     EditCounters& E = *d.edit;
     // An edit that failed (scratch exhausted, or an error raised while it ran) leaves the root as it
@@ -1157,13 +1175,10 @@ __device__ void ph_edit_end(const DevDag& d, char* scratch, uint32_t builder, ui
         if (!d.solo) // a subtree edit's overflow is reported by k_edit_spines, for that edit alone
             set_status(c, SVDAG_ERR_OOM);
     } else if ((E.count[d.leafLevel] != 0 || builder) && E.err == 0) {
-        const MergeLayout m = merge_layout_at(E.offM[E.startLevel], E.count[E.startLevel]);
-        const uint32_t r = reinterpret_cast<const uint32_t*>(scratch + m.rep)[0];
-        const uint32_t h = r == kEmptyRep ? kNone : reinterpret_cast<const uint32_t*>(scratch + m.handle)[r];
         if (tileOut)
-            *tileOut = h;
+            *tileOut = root;
         else
-            c->root = h;
+            c->root = root;
     }
     E.rootAfter = c->root;
     if (record) {
@@ -1182,6 +1197,15 @@ __device__ void ph_edit_end(const DevDag& d, char* scratch, uint32_t builder, ui
     }
 }
 
+// The handle of the edit's topmost node from its level's merge arrays.
+__device__ uint32_t merged_top(const DevDag& d, const char* scratch)
+{
+    const EditCounters& E = *d.edit;
+    const MergeLayout m = merge_layout_at(E.offM[E.startLevel], E.count[E.startLevel]);
+    const uint32_t r = reinterpret_cast<const uint32_t*>(scratch + m.rep)[0];
+    return r == kEmptyRep ? kNone : reinterpret_cast<const uint32_t*>(scratch + m.handle)[r];
+}
+
 __device__ void ph_reset_counters(const DevDag& d)
 {
     if (ph_block(d) != 0)
@@ -1191,59 +1215,38 @@ __device__ void ph_reset_counters(const DevDag& d)
         w[i] = 0;
 }
 
-// ---------------------------------------------------------------- kernel wrappers (one launch per phase)
-
-__global__ void k_edit_begin(DevDag d, EditQueue* q, char* scratch)
-{
-    if (q->eds) { // next editor of the batch into the slot
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(q->eds + q->cursor);
-        uint32_t* dst = reinterpret_cast<uint32_t*>(&q->slot);
-        for (uint32_t i = threadIdx.x; i < sizeof(DevEditor) / 4; i += blockDim.x)
-            dst[i] = src[i];
-        __syncwarp();
-    }
-    ph_reset_counters(d);
-    __syncwarp();
-    ph_edit_begin(d, q->slot, scratch);
-}
-template <uint32_t TOOL>
-__global__ void __launch_bounds__(256) k_build_level(DevDag d, const EditQueue* q, uint32_t level, char* scratch, unsigned long long scratchBytes)
-{
-    const DevEditor e = q->slot;
-    ph_build_level<TOOL>(d, e, level, scratch, scratchBytes);
-}
-template <uint32_t TOOL>
-__global__ void __launch_bounds__(256) k_build_leaves(DevDag d, const EditQueue* q, char* scratch, unsigned long long scratchBytes)
-{
-    const DevEditor e = q->slot;
-    ph_build_leaves<TOOL>(d, e, scratch, scratchBytes);
-}
-__global__ void __launch_bounds__(256) k_fix_level(DevDag d, uint32_t level, uint32_t builder, char* scratch)
-{
-    ph_fix_level(d, level, builder, scratch);
-}
-__global__ void __launch_bounds__(256) k_dedup_level(DevDag d, uint32_t level, char* scratch) { ph_dedup_level(d, level, scratch); }
-__global__ void __launch_bounds__(256) k_merge_level(DevDag d, uint32_t level, char* scratch) { ph_merge_level<false>(d, level, scratch); }
-template <int G>
-__global__ void __launch_bounds__(256) k_insert_level(DevDag d, DevTable t, uint32_t level, char* scratch)
-{
-    ph_insert_level<G>(d, t, level, scratch);
-}
-__global__ void k_edit_end(DevDag d, char* scratch, EditQueue* q)
-{
-    ph_edit_end(d, scratch, q->slot.builder, q->slot.tileOut, q->slot.record);
-    if (threadIdx.x == 0 && q->eds)
-        ++q->cursor;
-}
-
-// ---------------------------------------------------------------- persistent form
-// The persistent form for small edits: one CTA of 512 threads runs whole edits, one after another,
-// every phase above being a block-stride loop over the device-resident counts and the phases
-// separated by block barriers. Small SVOs thus cost one launch per batch instead of ~35 launches
-// per edit. All threads reach every barrier (phases only return early, never skip a barrier).
-
+// ---------------------------------------------------------------- narrow levels
+// Levels of few items are bound by latency: a phase over one item is a chain of dependent accesses,
+// and a launch of its own costs more than the phase. One block therefore runs all of an edit's narrow
+// levels: top-down with the level's work items and their nodes in shared memory (a child's words
+// are fetched when its header is, so a level costs one round trip to memory), bottom-up with the
+// items, the duplicate search and the children's handles in shared memory, the next level's items
+// loaded ahead, lookups and inserts separated by a barrier instead of published slot by slot (level
+// tables are touched by their level alone), and plain stores where one thread is the only writer.
+// kNarrow items is a level's limit: two passes of eight lanes per item over 512 threads. Measured against
+// a captured graph with one launch per phase: a stroke of radius 9 at depth 13 143 -> 70 us, a sphere
+// removal of radius 133 at depth 14 200 -> 117 us, 256 scattered small edits 2.8 -> 1.3 ms (their blocks
+// use the same code).
+constexpr uint32_t kNarrow = 128;
 constexpr uint32_t kBlockThreads = 512;
+constexpr uint32_t kNarrowTable = 512; // duplicate search of a narrow level, open addressing
 
+union NarrowShared {
+    struct {
+        WorkItem work[2][kNarrow];
+        uint4 node[2][kNarrow][3]; // words of the work item's node (a zero header without one)
+        uint32_t count[kMaxLevels + 1];
+    } build;
+    struct {
+        uint32_t items[kNarrow * 11]; // stride 11: odd, so that threads' rows fall in different banks
+        uint32_t handle[2][kNarrow]; // resolved handles of this level's and the child level's items
+        uint32_t table[kNarrowTable]; // item index + 1
+        DevTable tables[kMaxLevels];
+        uint32_t full[kMaxLevels], reps[kMaxLevels], ran[kMaxLevels], added;
+    } merge;
+};
+
+// GPU-clock stamps at the phase barriers (svdag_last_edit_phase_times).
 __device__ __forceinline__ void stamp(const DevDag& d, uint32_t& k)
 {
     if (!d.solo && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1255,70 +1258,486 @@ __device__ __forceinline__ void stamp(const DevDag& d, uint32_t& k)
     }
 }
 
-template <uint32_t TOOL, bool SHARED = false>
-__device__ __forceinline__ void block_edit(const DevDag& d, const DevEditor& ed, char* scratch, unsigned long long scratchBytes,
-    EditRecord* record)
+// Top-down phases of the levels from the edit's first one while they are below `endLevel` and narrow,
+// in one block (all threads call); returns the first level left. Its work items are in scratch, as
+// ph_build_level leaves them; the intermediate items of every level are written there.
+template <uint32_t TOOL>
+__device__ uint32_t narrow_build(const DevDag& d, const DevEditor& e, uint32_t endLevel, char* scratch, unsigned long long scratchBytes,
+    NarrowShared& sh, uint32_t& stampAt)
+{
+    EditCounters& E = *d.edit;
+    uint32_t level = e.startLevel;
+    if constexpr (TOOL == SVDAG_TOOL_COPY) { // its work items carry the source parents: the plain phases, in one block
+        DevDag one = d;
+        one.solo = 1;
+        for (; level < endLevel && E.count[level] <= kNarrow; ++level) {
+            ph_build_level<TOOL>(one, e, level, scratch, scratchBytes);
+            __syncthreads();
+            stamp(d, stampAt);
+        }
+        return level;
+    }
+    auto& B = sh.build;
+    const uint32_t lane = threadIdx.x & 31u, c = lane & 7u, grp = lane >> 3;
+    const uint32_t warps = blockDim.x >> 5;
+    for (uint32_t l = threadIdx.x; l <= kMaxLevels; l += blockDim.x)
+        B.count[l] = 0;
+    if (threadIdx.x == 0)
+        B.work[0][0] = *reinterpret_cast<const WorkItem*>(scratch);
+    if (threadIdx.x < 3) {
+        const uint32_t h = reinterpret_cast<const WorkItem*>(scratch)->handle;
+        B.node[0][0][threadIdx.x] = h == kNone ? make_uint4(0, 0, 0, 0) : reinterpret_cast<const uint4*>(item_ptr(d, h))[threadIdx.x];
+    }
+    __syncthreads();
+    unsigned long long offW = 0, edited = 0;
+    uint32_t n = 1, cur = 0, oldRead = 0;
+    for (; level < endLevel && n <= kNarrow; ++level) {
+        const unsigned long long offN = align256(offW + n * 16ull), offWn = align256(offN + (unsigned long long)n * 4 * kItemStride);
+        if (threadIdx.x == 0) {
+            E.offN[level] = offN;
+            E.offW[level + 1] = offWn;
+        }
+        const uint32_t childLevel = level + 1, childDepth = d.levels - childLevel;
+        const bool fits = offN + (unsigned long long)n * 4 * kItemStride <= scratchBytes;
+        if (!fits && threadIdx.x == 0)
+            E.overflow = 1;
+        for (uint32_t base = (threadIdx.x >> 5) * 4; fits && base < n; base += warps * 4) {
+            const uint32_t i = base + grp;
+            const bool active = i < n;
+            WorkItem w { 0, 0, 0, kNone };
+            if (active)
+                w = B.work[cur][i];
+            uint32_t child = kNone, state = ST_EMPTY, fillMat = 0;
+            uint4 cw[3] = {};
+            if (active && w.handle != kNone) {
+                const uint32_t* node = reinterpret_cast<const uint32_t*>(B.node[cur][i]);
+                const uint32_t mask = node[0] & 0xFFu;
+                if (mask & (1u << c)) {
+                    child = node[1 + __popc(mask & ((1u << c) - 1u))];
+                    state = ST_PARTIAL;
+                    if (childLevel != d.leafLevel) { // every valid handle has 16 readable words
+                        const uint4* p = reinterpret_cast<const uint4*>(item_ptr(d, child));
+                        cw[0] = p[0];
+                        cw[1] = p[1];
+                        cw[2] = p[2];
+                        if ((cw[0].x >> 8) & 1u)
+                            state = ST_FILLED;
+                    }
+                }
+                if (c == 0)
+                    ++oldRead;
+            }
+            const uint32_t cx = (w.x << 1) | ((c >> 2) & 1u), cy = (w.y << 1) | ((c >> 1) & 1u), cz = (w.z << 1) | (c & 1u);
+            uint32_t op = OP_KEEP;
+            if (active)
+                op = should_edit<TOOL>(e, cx, cy, cz, childDepth, state, fillMat);
+            if (op == OP_FILL || op == OP_EMPTY)
+                edited += 1ull << (3 * childDepth);
+            const bool subdivide = op == OP_SUBDIVIDE;
+            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, subdivide);
+            uint32_t idx0 = 0;
+            if (lane == 0 && bal)
+                idx0 = atomicAdd(&B.count[childLevel], __popc(bal));
+            idx0 = __shfl_sync(0xFFFFFFFFu, idx0, 0);
+            if (subdivide) {
+                const uint32_t idx = idx0 + __popc(bal & ((1u << lane) - 1u));
+                const WorkItem next { cx, cy, cz, child };
+                const unsigned long long at = offWn + idx * 16ull;
+                if (at + 16ull <= scratchBytes)
+                    *reinterpret_cast<WorkItem*>(scratch + at) = next;
+                else
+                    atomicExch(&E.overflow, 1u);
+                if (idx < kNarrow) {
+                    B.work[cur ^ 1][idx] = next;
+                    B.node[cur ^ 1][idx][0] = cw[0];
+                    B.node[cur ^ 1][idx][1] = cw[1];
+                    B.node[cur ^ 1][idx][2] = cw[2];
+                }
+                child = idx;
+            } else if (op == OP_EMPTY) {
+                child = kNone;
+            } else if (op == OP_FILL) {
+                child = kFillMarker | fillMat;
+            }
+            const uint32_t present = __ballot_sync(0xFFFFFFFFu, active && child != kNone);
+            const uint32_t outMask = (present >> (grp * 8)) & 0xFFu, intMask = (bal >> (grp * 8)) & 0xFFu;
+            if (active) { // the item, as ph_build_level writes it
+                uint32_t* node = reinterpret_cast<uint32_t*>(scratch + offN) + (size_t)i * kItemStride;
+                if (c == 0) {
+                    node[0] = outMask ? (outMask | (intMask << 13)) : 0u;
+                    node[9] = 0;
+                }
+                if (child != kNone)
+                    node[1 + __popc(outMask & ((1u << c) - 1u))] = child;
+                if (c >= __popc(outMask))
+                    node[1 + c] = 0;
+            }
+        }
+        __syncthreads();
+        n = B.count[childLevel];
+        if (threadIdx.x == 0)
+            E.count[childLevel] = n;
+        stamp(d, stampAt);
+        cur ^= 1u;
+        offW = offWn;
+        if (!fits)
+            return endLevel; // the later phases see the overflow
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        edited += __shfl_xor_sync(0xFFFFFFFFu, edited, o);
+        oldRead += __shfl_xor_sync(0xFFFFFFFFu, oldRead, o);
+    }
+    if (lane == 0) {
+        if (edited)
+            atomicAdd(&E.edited, edited);
+        if (oldRead)
+            atomicAdd(&E.oldRead, (unsigned long long)oldRead);
+    }
+    __syncthreads();
+    return level;
+}
+
+// Bottom-up phases of the levels fromLevel .. the edit's first one, each of at most kNarrow items, in one
+// block (all threads call, after the merges of the levels below); returns the topmost node's handle to
+// every thread. SHARED: other blocks insert into the same tables.
+template <bool SHARED>
+__device__ uint32_t narrow_merge(const DevDag& d, uint32_t fromLevel, char* scratch, NarrowShared& sh, uint32_t& stampAt)
+{
+    EditCounters& E = *d.edit;
+    if (!merge_live(d))
+        return kNone;
+    for (uint32_t l = E.startLevel; l <= fromLevel; ++l)
+        if (E.count[l] > kNarrow) { // the caller's bounds rule this out
+            set_status(d.ctl, SVDAG_ERR_CORRUPT);
+            return kNone;
+        }
+    auto& M = sh.merge;
+    const uint32_t LL = d.leafLevel, tid = threadIdx.x, startLevel = E.startLevel, builder = E.builder;
+    Grp<1> g;
+    for (uint32_t k = tid; k < sizeof(M.tables) / 4; k += blockDim.x)
+        reinterpret_cast<uint32_t*>(M.tables)[k] = reinterpret_cast<const uint32_t*>(d.ctl->tables)[k];
+    for (uint32_t l = tid; l < kMaxLevels; l += blockDim.x) {
+        M.full[l] = l == fromLevel + 1 || (l == LL && fromLevel == LL) ? E.ffCount[l] : 0u; // the leaf phase counts its own
+        M.ran[l] = l == fromLevel + 1 ? E.ffRan[l] : 0u;
+        M.reps[l] = 0;
+    }
+    if (tid == 0)
+        M.added = 0;
+    for (uint32_t k = tid; k < kNarrowTable; k += blockDim.x)
+        M.table[k] = 0;
+    const auto load_item = [&](uint32_t level, uint32_t n, uint32_t (&w)[kItemStride]) {
+        const uint32_t* it = reinterpret_cast<const uint32_t*>(scratch + E.offN[level]) + (size_t)tid * kItemStride;
+#pragma unroll
+        for (uint32_t j = 0; j < kItemStride; ++j)
+            w[j] = tid < n ? it[j] : 0u;
+    };
+    uint32_t n = E.count[fromLevel], cur = 0, added = 0;
+    uint32_t next[kItemStride];
+    load_item(fromLevel, n, next);
+    __syncthreads();
+    for (int li = (int)fromLevel; li >= (int)startLevel; --li) {
+        const uint32_t level = (uint32_t)li;
+        const bool isLeaf = level == LL;
+        const bool gate = !isLeaf && (builder || ((level + 1 == LL || M.ran[level + 1] != 0) && M.full[level + 1] > 0)); // discovery_gate
+        Key<1> key;
+#pragma unroll
+        for (uint32_t j = 0; j < kItemStride; ++j)
+            key.w[j] = next[j];
+        const uint32_t nAbove = level > startLevel ? E.count[level - 1] : 0u;
+        if (level > startLevel)
+            load_item(level - 1, nAbove, next);
+        bool live = tid < n, full = false;
+        if (live && !isLeaf) {
+            if (level == fromLevel) {
+                const MergeLayout ch = merge_layout_at(E.offM[level + 1], E.count[level + 1]);
+                full = fix_node(d, level, gate,
+                    ArrayChildren { reinterpret_cast<const uint32_t*>(scratch + ch.rep), reinterpret_cast<const uint32_t*>(scratch + ch.handle) },
+                    key.w);
+            } else {
+                full = fix_node(d, level, gate, ResolvedChildren { M.handle[cur ^ 1u] }, key.w);
+            }
+        }
+        if (live && (isLeaf ? (key.w[0] == 0 && key.w[1] == 0) : (key.w[0] & 0xFFu) == 0)) {
+            M.handle[cur][tid] = kNone;
+            live = false;
+        }
+        uint32_t rep = tid;
+        if (live) {
+            key.n = isLeaf ? dev_leaf_words(key.w[0], key.w[1]) : dev_node_words(key.w[0]);
+            hash_words(key.w, key.n, key.ha, key.hb);
+        }
+        if (n > 1) { // duplicates within the level: every thread's words, then one table of indices
+            uint32_t* row = M.items + tid * 11u;
+            if (live) {
+#pragma unroll
+                for (uint32_t j = 0; j < kItemStride; ++j)
+                    row[j] = j < key.n ? key.w[j] : 0u;
+            }
+            __syncthreads();
+            if (live) {
+                uint32_t slot = key.ha & (kNarrowTable - 1u);
+                for (uint32_t probe = 0; probe < kNarrowTable; ++probe) {
+                    const uint32_t was = atomicCAS(&M.table[slot], 0u, tid + 1u);
+                    if (was == 0)
+                        break;
+                    const uint32_t* other = M.items + (was - 1u) * 11u;
+                    bool same = true;
+#pragma unroll
+                    for (uint32_t j = 0; j < kItemStride; ++j)
+                        same &= other[j] == (j < key.n ? key.w[j] : 0u);
+                    if (same) {
+                        rep = was - 1u;
+                        break;
+                    }
+                    slot = (slot + 1u) & (kNarrowTable - 1u);
+                }
+            }
+        }
+        const bool mine = live && rep == tid;
+        uint32_t h = kNone;
+        bool inserted = false;
+        if constexpr (SHARED) {
+            if (n > 1)
+                __syncthreads(); // the duplicate search is over before its table is cleared below
+            if (mine)
+                h = table_find_or_insert<1, kInsertShared>(g, d, M.tables[level], key, inserted);
+        } else if (n == 1) {
+            if (mine) {
+                Probed<1> at;
+                bool ok;
+                h = table_probe<1>(g, d, M.tables[level], key, at, ok);
+                if (h == kNone && ok) {
+                    h = table_insert_probed<1, kSole>(g, d, M.tables[level], key, at);
+                    inserted = h != kNone;
+                }
+            }
+        } else {
+            Probed<1> at;
+            bool ok = false;
+            if (mine)
+                h = table_probe<1>(g, d, M.tables[level], key, at, ok);
+            __syncthreads(); // lookups are over: inserts need not hide their unfinished items
+            if (mine && h == kNone && ok) {
+                h = table_insert_probed<1, kQuiet>(g, d, M.tables[level], key, at);
+                inserted = h != kNone;
+            }
+        }
+        added += inserted ? 1u : 0u;
+        if (mine)
+            M.handle[cur][tid] = h;
+        if (mine && n > 1)
+            atomicAdd(&M.reps[level], 1u);
+        if (full)
+            atomicAdd(&M.full[level], 1u);
+        if (tid == 0) {
+            if (!isLeaf)
+                M.ran[level] = gate ? 1u : 0u;
+            if (n == 1 && mine)
+                M.reps[level] = 1;
+        }
+        if (n > 1) {
+            for (uint32_t k = tid; k < kNarrowTable; k += blockDim.x)
+                M.table[k] = 0;
+            __syncthreads();
+            if (live && rep != tid)
+                M.handle[cur][tid] = M.handle[cur][rep];
+        }
+        __syncthreads();
+        stamp(d, stampAt);
+        cur ^= 1u;
+        n = nAbove;
+    }
+    if (added)
+        atomicAdd(&M.added, added);
+    __syncthreads();
+    for (uint32_t l = startLevel + tid; l <= fromLevel; l += blockDim.x) {
+        E.repCount[l] = M.reps[l];
+        if (l != LL) {
+            E.ffCount[l] = M.full[l];
+            E.ffRan[l] = M.ran[l];
+        }
+    }
+    const uint32_t top = M.handle[cur ^ 1u][0];
+    if (tid == 0)
+        E.added += M.added;
+    __threadfence(); // the inserted items are visible before the root that reaches them
+    __syncthreads();
+    return top;
+}
+
+// ---------------------------------------------------------------- kernel wrappers
+// An edit is the chain of launches k_edit_top (begin and the narrow levels from the top), one
+// k_build_level for each wide level, k_build_leaves, one k_merge_level for each wide level, k_edit_bottom
+// (the narrow levels and the end). Each launch may become resident while its predecessor still runs
+// (programmatic dependent launch) and waits for its end before it touches memory.
+
+__device__ __forceinline__ void chain_wait()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <uint32_t TOOL>
+__global__ void __launch_bounds__(kBlockThreads, 1) k_edit_top(DevDag d, const __grid_constant__ DevEditor e, uint32_t endLevel, char* scratch,
+    unsigned long long scratchBytes)
+{
+    __shared__ NarrowShared sh;
+    chain_wait();
+    ph_reset_counters(d);
+    __syncthreads();
+    ph_edit_begin(d, e, scratch);
+    __syncthreads();
+    uint32_t k = 64; // no stamps
+    if (narrow_build<TOOL>(d, e, endLevel, scratch, scratchBytes, sh, k) < endLevel && threadIdx.x == 0) { // ruled out by the caller's bounds
+        set_status(d.ctl, SVDAG_ERR_CORRUPT);
+        d.edit->overflow = 1;
+    }
+}
+template <uint32_t TOOL>
+__global__ void __launch_bounds__(256) k_build_level(DevDag d, const __grid_constant__ DevEditor e, uint32_t level, char* scratch,
+    unsigned long long scratchBytes)
+{
+    chain_wait();
+    ph_build_level<TOOL>(d, e, level, scratch, scratchBytes);
+}
+template <uint32_t TOOL>
+__global__ void __launch_bounds__(256) k_build_leaves(DevDag d, const __grid_constant__ DevEditor e, char* scratch, unsigned long long scratchBytes)
+{
+    chain_wait();
+    ph_build_leaves<TOOL>(d, e, scratch, scratchBytes);
+}
+__global__ void __launch_bounds__(256) k_fix_level(DevDag d, uint32_t level, uint32_t builder, char* scratch)
+{
+    ph_fix_level(d, level, builder, scratch);
+}
+__global__ void __launch_bounds__(256) k_dedup_level(DevDag d, uint32_t level, char* scratch) { ph_dedup_level(d, level, scratch); }
+__global__ void __launch_bounds__(256, 4) k_merge_level(DevDag d, uint32_t level, char* scratch)
+{
+    chain_wait();
+    ph_merge_level<false>(d, level, scratch);
+}
+template <int G>
+__global__ void __launch_bounds__(256) k_insert_level(DevDag d, DevTable t, uint32_t level, char* scratch)
+{
+    ph_insert_level<G>(d, t, level, scratch);
+}
+// `endLevel` as in k_edit_top: the levels below it are narrow (none when it is the edit's first level: the
+// merge launches did them all).
+__global__ void __launch_bounds__(kBlockThreads, 1) k_edit_bottom(DevDag d, uint32_t endLevel, uint32_t startLevel, uint32_t builder,
+    uint32_t* tileOut, EditRecord* record, char* scratch)
+{
+    __shared__ NarrowShared sh;
+    chain_wait();
+    uint32_t k = 64, root = kNone; // no stamps
+    if (endLevel > startLevel)
+        root = narrow_merge<false>(d, endLevel - 1u, scratch, sh, k);
+    else if (merge_live(d))
+        root = merged_top(d, scratch);
+    if (threadIdx.x == 0)
+        edit_end(d, root, builder, tileOut, record);
+}
+
+// ---------------------------------------------------------------- persistent form
+// The persistent form for small edits: one CTA of 512 threads runs whole edits, one after another:
+// the narrow levels as above, the others as block-stride loops over the device-resident counts, the
+// phases separated by block barriers. Small SVOs thus cost one launch per batch. All threads reach every
+// barrier (phases only return early, never skip a barrier).
+
+// Top-down phases and the leaves; returns the first level that narrow_build left.
+template <uint32_t TOOL>
+__device__ __forceinline__ uint32_t block_build(const DevDag& d, const DevEditor& ed, char* scratch, unsigned long long scratchBytes,
+    NarrowShared& sh, uint32_t& stampAt)
 {
     const uint32_t LL = d.leafLevel;
-    uint32_t k = 0;
+    const uint32_t wide = narrow_build<TOOL>(d, ed, LL, scratch, scratchBytes, sh, stampAt);
+    for (uint32_t level = wide; level < LL; ++level) {
+        ph_build_level<TOOL>(d, ed, level, scratch, scratchBytes);
+        __syncthreads();
+        stamp(d, stampAt);
+    }
+    ph_build_leaves<TOOL>(d, ed, scratch, scratchBytes);
+    __syncthreads();
+    stamp(d, stampAt);
+    return wide;
+}
+
+// One whole edit in this block. SUBTREES: an edit of a group (the tools that qualify, shared tables).
+template <bool SUBTREES>
+__device__ __forceinline__ void block_edit(const DevDag& d, const DevEditor& ed, char* scratch, unsigned long long scratchBytes,
+    EditRecord* record, NarrowShared& sh)
+{
+    const uint32_t LL = d.leafLevel;
+    uint32_t k = 0, wide = LL;
     stamp(d, k);
     ph_reset_counters(d);
     __syncthreads();
     ph_edit_begin(d, ed, scratch);
     __syncthreads();
     stamp(d, k);
-    for (uint32_t level = 0; level < LL; ++level) {
-        ph_build_level<TOOL>(d, ed, level, scratch, scratchBytes);
+    switch (ed.tool) {
+    case SVDAG_TOOL_SPHERE_ADD:
+        wide = block_build<SVDAG_TOOL_SPHERE_ADD>(d, ed, scratch, scratchBytes, sh, k);
+        break;
+    case SVDAG_TOOL_SPHERE_REMOVE:
+        wide = block_build<SVDAG_TOOL_SPHERE_REMOVE>(d, ed, scratch, scratchBytes, sh, k);
+        break;
+    case SVDAG_TOOL_BOX_ADD:
+        wide = block_build<SVDAG_TOOL_BOX_ADD>(d, ed, scratch, scratchBytes, sh, k);
+        break;
+    case SVDAG_TOOL_BOX_REMOVE:
+        wide = block_build<SVDAG_TOOL_BOX_REMOVE>(d, ed, scratch, scratchBytes, sh, k);
+        break;
+    case SVDAG_TOOL_SPHERE_PAINT:
+        wide = block_build<SVDAG_TOOL_SPHERE_PAINT>(d, ed, scratch, scratchBytes, sh, k);
+        break;
+    case SVDAG_TOOL_BOX_PAINT_NOISE:
+        wide = block_build<SVDAG_TOOL_BOX_PAINT_NOISE>(d, ed, scratch, scratchBytes, sh, k);
+        break;
+    case SVDAG_TOOL_COPY:
+        if constexpr (!SUBTREES)
+            wide = block_build<SVDAG_TOOL_COPY>(d, ed, scratch, scratchBytes, sh, k);
+        break;
+    case SVDAG_TOOL_SPHERE_ERODE:
+        if constexpr (!SUBTREES)
+            wide = block_build<SVDAG_TOOL_SPHERE_ERODE>(d, ed, scratch, scratchBytes, sh, k);
+        break;
+    default:
+        break;
+    }
+    const bool allNarrow = wide == LL && d.edit->count[LL] <= kNarrow;
+    for (int level = (int)LL; !allNarrow && level >= (int)wide; --level) {
+        ph_merge_level<SUBTREES>(d, (uint32_t)level, scratch);
         __syncthreads();
         stamp(d, k);
     }
-    ph_build_leaves<TOOL>(d, ed, scratch, scratchBytes);
-    __syncthreads();
-    stamp(d, k);
-    for (int level = (int)LL; level >= 0; --level) {
-        ph_merge_level<SHARED>(d, (uint32_t)level, scratch);
-        __syncthreads();
-        stamp(d, k);
-    }
-    ph_edit_end(d, scratch, ed.builder, ed.tileOut, record);
+    uint32_t root = kNone;
+    if (allNarrow || wide > ed.startLevel)
+        root = narrow_merge<SUBTREES>(d, allNarrow ? LL : wide - 1u, scratch, sh, k);
+    else if (merge_live(d))
+        root = merged_top(d, scratch);
+    if (threadIdx.x == 0)
+        edit_end(d, root, ed.builder, ed.tileOut, record);
     __syncthreads();
     stamp(d, k);
 }
 
-__global__ void __launch_bounds__(kBlockThreads, 1) k_edit_block(DevDag d, DevEditor single, const DevEditor* eds, uint32_t numEdits,
-    char* scratch, unsigned long long scratchBytes, EditRecord* records)
+// An editor in shared memory: a copy in registers or on the stack costs the whole block's phases.
+__device__ __forceinline__ void load_editor(DevEditor& to, const DevEditor& from)
 {
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < sizeof(DevEditor) / 4; i += blockDim.x)
+        reinterpret_cast<uint32_t*>(&to)[i] = reinterpret_cast<const uint32_t*>(&from)[i];
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kBlockThreads, 1) k_edit_block(DevDag d, const __grid_constant__ DevEditor single, const DevEditor* eds,
+    uint32_t numEdits, char* scratch, unsigned long long scratchBytes, EditRecord* records)
+{
+    __shared__ NarrowShared sh;
+    __shared__ DevEditor ed;
     for (uint32_t k = 0; k < numEdits; ++k) {
-        const DevEditor ed = eds ? eds[k] : single;
-        EditRecord* rec = records ? &records[k] : nullptr;
-        switch (ed.tool) {
-        case SVDAG_TOOL_SPHERE_ADD:
-            block_edit<SVDAG_TOOL_SPHERE_ADD>(d, ed, scratch, scratchBytes, rec);
-            break;
-        case SVDAG_TOOL_SPHERE_REMOVE:
-            block_edit<SVDAG_TOOL_SPHERE_REMOVE>(d, ed, scratch, scratchBytes, rec);
-            break;
-        case SVDAG_TOOL_BOX_ADD:
-            block_edit<SVDAG_TOOL_BOX_ADD>(d, ed, scratch, scratchBytes, rec);
-            break;
-        case SVDAG_TOOL_BOX_REMOVE:
-            block_edit<SVDAG_TOOL_BOX_REMOVE>(d, ed, scratch, scratchBytes, rec);
-            break;
-        case SVDAG_TOOL_SPHERE_PAINT:
-            block_edit<SVDAG_TOOL_SPHERE_PAINT>(d, ed, scratch, scratchBytes, rec);
-            break;
-        case SVDAG_TOOL_COPY:
-            block_edit<SVDAG_TOOL_COPY>(d, ed, scratch, scratchBytes, rec);
-            break;
-        case SVDAG_TOOL_BOX_PAINT_NOISE:
-            block_edit<SVDAG_TOOL_BOX_PAINT_NOISE>(d, ed, scratch, scratchBytes, rec);
-            break;
-        case SVDAG_TOOL_SPHERE_ERODE:
-            block_edit<SVDAG_TOOL_SPHERE_ERODE>(d, ed, scratch, scratchBytes, rec);
-            break;
-        default:
-            break;
-        }
+        load_editor(ed, eds ? eds[k] : single);
+        block_edit<false>(d, ed, scratch, scratchBytes, records ? &records[k] : nullptr, sh);
     }
 }
 
@@ -1330,36 +1749,16 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_edit_block(DevDag d, DevEd
 __global__ void __launch_bounds__(kBlockThreads, 1) k_edit_subtrees(DevDag d, const DevEditor* eds, uint32_t numEdits, char* parts,
     unsigned long long partBytes, EditCounters* counters)
 {
+    __shared__ NarrowShared sh;
     const uint32_t k = blockIdx.x;
     if (k >= numEdits)
         return;
     DevDag dk = d;
     dk.edit = counters + k;
     dk.solo = 1;
-    const DevEditor ed = eds[k];
-    char* scratch = parts + (unsigned long long)k * partBytes;
-    switch (ed.tool) {
-    case SVDAG_TOOL_SPHERE_ADD:
-        block_edit<SVDAG_TOOL_SPHERE_ADD, true>(dk, ed, scratch, partBytes, nullptr);
-        break;
-    case SVDAG_TOOL_SPHERE_REMOVE:
-        block_edit<SVDAG_TOOL_SPHERE_REMOVE, true>(dk, ed, scratch, partBytes, nullptr);
-        break;
-    case SVDAG_TOOL_BOX_ADD:
-        block_edit<SVDAG_TOOL_BOX_ADD, true>(dk, ed, scratch, partBytes, nullptr);
-        break;
-    case SVDAG_TOOL_BOX_REMOVE:
-        block_edit<SVDAG_TOOL_BOX_REMOVE, true>(dk, ed, scratch, partBytes, nullptr);
-        break;
-    case SVDAG_TOOL_SPHERE_PAINT:
-        block_edit<SVDAG_TOOL_SPHERE_PAINT, true>(dk, ed, scratch, partBytes, nullptr);
-        break;
-    case SVDAG_TOOL_BOX_PAINT_NOISE:
-        block_edit<SVDAG_TOOL_BOX_PAINT_NOISE, true>(dk, ed, scratch, partBytes, nullptr);
-        break;
-    default:
-        break;
-    }
+    __shared__ DevEditor ed;
+    load_editor(ed, eds[k]);
+    block_edit<true>(dk, ed, parts + (unsigned long long)k * partBytes, partBytes, nullptr, sh);
 }
 
 // Commits a group of subtree edits: each edit's path from its node up to the root (levels
@@ -1464,9 +1863,8 @@ __global__ void __launch_bounds__(1024) k_edit_spines(DevDag d, const DevEditor*
                 if ((mask >> b) & 1u)
                     w[1 + j++] = b == ck ? 0u : kid[b];
             w[0] = mask | (1u << (13 + ck));
-            const uint32_t childHandle = ver[l + 1][k];
-            const uint32_t regRep[1] = { childHandle == kNone ? kEmptyRep : 0u }, regHandle[1] = { childHandle };
-            const uint32_t hn = merge_single<kInsertShared>(dk, l, w, regRep, regHandle, g, added);
+            const uint32_t childHandle[1] = { ver[l + 1][k] };
+            const uint32_t hn = merge_single<kInsertShared>(dk, l, w, childHandle, g, added);
             if (hn == kNone && (w[0] & 0xFFu) != 0) // not emptied: the insert failed
                 atomicMin(&failAt, k);
             ver[l][k] = hn;
@@ -1596,47 +1994,95 @@ DevEditor make_editor(const svdag_ctx* ctx, const svdag_edit& e)
     return d;
 }
 
-template <uint32_t TOOL>
-svdag_status launch_build(svdag_ctx* ctx, cudaStream_t s)
+// One launch of an edit's chain; `dependent` lets it become resident while its predecessor runs.
+template <class... Params, class... Args>
+svdag_status launch_chained(void (*kernel)(Params...), int grid, int block, bool dependent, cudaStream_t s, const Args&... args)
 {
-    const DevDag d = ctx->dag();
-    const EditQueue* q = ctx->queue;
-    const uint32_t LL = d.leafLevel;
-    for (uint32_t level = 0; level < LL; ++level) {
-        const unsigned long long bound = level < 8 ? (1ull << (3 * level)) : (1ull << 24);
-        k_build_level<TOOL><<<grid_for(ctx, bound * 8, 256), 256, 0, s>>>(d, q, level, ctx->scratch, ctx->scratchBytes);
-    }
-    const unsigned long long bound = LL < 8 ? (1ull << (3 * LL)) : (1ull << 24);
-    k_build_leaves<TOOL><<<grid_for(ctx, bound * 32, 256), 256, 0, s>>>(d, q, ctx->scratch, ctx->scratchBytes);
-    SVDAG_CUDA(cudaGetLastError());
+    cudaLaunchConfig_t cfg {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = s;
+    cudaLaunchAttribute attr {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    SVDAG_CUDA(cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
     return SVDAG_OK;
 }
 
-svdag_status launch_build_any(svdag_ctx* ctx, uint32_t tool, cudaStream_t s)
+// Upper bounds of an edit's SVO items per level (from its first level on): the nodes its footprint, grown
+// by two voxels, can meet.
+struct LevelBounds {
+    unsigned long long n[kMaxLevels];
+};
+LevelBounds level_bounds(const svdag_ctx* ctx, const DevEditor& e)
 {
-    switch (tool) {
+    float lo[3], hi[3];
+    bool box = true;
+    switch (e.tool) {
     case SVDAG_TOOL_SPHERE_ADD:
-        return launch_build<SVDAG_TOOL_SPHERE_ADD>(ctx, s);
     case SVDAG_TOOL_SPHERE_REMOVE:
-        return launch_build<SVDAG_TOOL_SPHERE_REMOVE>(ctx, s);
-    case SVDAG_TOOL_BOX_ADD:
-        return launch_build<SVDAG_TOOL_BOX_ADD>(ctx, s);
-    case SVDAG_TOOL_BOX_REMOVE:
-        return launch_build<SVDAG_TOOL_BOX_REMOVE>(ctx, s);
     case SVDAG_TOOL_SPHERE_PAINT:
-        return launch_build<SVDAG_TOOL_SPHERE_PAINT>(ctx, s);
-    case SVDAG_TOOL_COPY:
-        return launch_build<SVDAG_TOOL_COPY>(ctx, s);
-    case SVDAG_TOOL_BOX_PAINT_NOISE:
-        return launch_build<SVDAG_TOOL_BOX_PAINT_NOISE>(ctx, s);
     case SVDAG_TOOL_SPHERE_ERODE:
-        return launch_build<SVDAG_TOOL_SPHERE_ERODE>(ctx, s);
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = e.center[a] - e.radius;
+            hi[a] = e.center[a] + e.radius;
+        }
+        break;
     case kToolTerrain:
-        return launch_build<kToolTerrain>(ctx, s);
+        box = false;
+        break;
     default:
-        return SVDAG_ERR_INVALID;
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = e.bmin[a];
+            hi[a] = e.bmax[a];
+        }
+        break;
     }
+    LevelBounds b {};
+    const double g = (double)(1ull << ctx->cfg.levels);
+    for (uint32_t l = e.startLevel; l <= ctx->cfg.levels - 2; ++l) {
+        const uint32_t down = l - e.startLevel;
+        unsigned long long n = down < 16 ? 1ull << (3 * down) : 1ull << 48;
+        if (box) {
+            const double cell = (double)(1ull << (ctx->cfg.levels - l));
+            unsigned long long cells = 1;
+            for (int a = 0; a < 3; ++a) {
+                const double first = std::floor(std::min(std::max((double)lo[a] - 2.0, 0.0), g - 1.0) / cell);
+                const double last = std::floor(std::min(std::max((double)hi[a] + 2.0, 0.0), g - 1.0) / cell);
+                cells *= (unsigned long long)(last - first) + 1ull;
+            }
+            n = std::min(n, cells);
+        }
+        b.n[l] = n;
+    }
+    return b;
 }
+
+// The launches of one editor.
+template <uint32_t TOOL>
+svdag_status launch_edit(svdag_ctx* ctx, const DevEditor& e, EditRecord* record, cudaStream_t s)
+{
+    const DevDag d = ctx->dag();
+    const uint32_t LL = d.leafLevel;
+    const LevelBounds b = level_bounds(ctx, e);
+    // [startLevel, end): the levels that are narrow from the top (with SVDAG_FLAG_PHASE_KERNELS none are
+    // run together, so that every level's phases are launches of their own)
+    uint32_t end = e.startLevel;
+    while (!(ctx->cfg.flags & SVDAG_FLAG_PHASE_KERNELS) && end <= LL && b.n[end] <= kNarrow)
+        ++end;
+    const uint32_t firstWide = std::min(end, LL);
+    SVDAG_TRY(launch_chained(k_edit_top<TOOL>, 1, kBlockThreads, false, s, d, e, firstWide, ctx->scratch, ctx->scratchBytes));
+    for (uint32_t level = firstWide; level < LL; ++level)
+        SVDAG_TRY(launch_chained(k_build_level<TOOL>, grid_for(ctx, b.n[level] * 8, 256), 256, true, s, d, e, level, ctx->scratch, ctx->scratchBytes));
+    SVDAG_TRY(launch_chained(k_build_leaves<TOOL>, grid_for(ctx, b.n[LL] * 32, 256), 256, true, s, d, e, ctx->scratch, ctx->scratchBytes));
+    for (int level = (int)LL; level >= (int)end; --level)
+        SVDAG_TRY(launch_chained(k_merge_level, grid_for(ctx, b.n[level], 256), 256, true, s, d, (uint32_t)level, ctx->scratch));
+    return launch_chained(k_edit_bottom, 1, kBlockThreads, true, s, d, end, e.startLevel, e.builder, e.tileOut, record, ctx->scratch);
+}
+
+unsigned long long level_bound(uint32_t level) { return level < 8 ? (1ull << (3 * level)) : (1ull << 24); }
 
 svdag_status launch_insert(svdag_ctx* ctx, uint32_t level, unsigned long long bound, cudaStream_t s)
 {
@@ -1668,68 +2114,33 @@ svdag_status launch_insert(svdag_ctx* ctx, uint32_t level, unsigned long long bo
     return SVDAG_OK;
 }
 
-unsigned long long level_bound(uint32_t level) { return level < 8 ? (1ull << (3 * level)) : (1ull << 24); }
-
 } // namespace
 
-// The phases of the editor in the queue slot, one launch each.
-svdag_status launch_phases(svdag_ctx* ctx, uint32_t tool, cudaStream_t s)
+// One editor, passed to its launches by value.
+svdag_status launch_pipeline(svdag_ctx* ctx, const DevEditor& ed, cudaStream_t s, EditRecord* record)
 {
-    const DevDag d = ctx->dag();
-    k_edit_begin<<<1, 32, 0, s>>>(d, ctx->queue, ctx->scratch);
-    SVDAG_TRY(launch_build_any(ctx, tool, s));
-    const uint32_t LL = d.leafLevel;
-    for (int level = (int)LL; level >= 0; --level)
-        k_merge_level<<<grid_for(ctx, level_bound(level), 256), 256, 0, s>>>(d, level, ctx->scratch);
-    k_edit_end<<<1, 32, 0, s>>>(d, ctx->scratch, ctx->queue);
-    SVDAG_CUDA(cudaGetLastError());
-    return SVDAG_OK;
-}
-
-// Runs the editor in the queue slot: through the tool's CUDA graph of the phase launches (captured
-// on first use), or launch by launch with SVDAG_FLAG_PHASE_KERNELS and while a scene build has
-// lent part of the scratch arena.
-svdag_status run_phases(svdag_ctx* ctx, uint32_t tool, cudaStream_t s, bool graphOk)
-{
-    const int g = tool == kToolTerrain ? kNumGraphs - 1 : (int)tool;
-    if (!graphOk || (ctx->cfg.flags & SVDAG_FLAG_PHASE_KERNELS) || g < 0 || g >= kNumGraphs)
-        return launch_phases(ctx, tool, s);
-    if (!ctx->graphs[g]) {
-        cudaStream_t cs;
-        SVDAG_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-        cudaGraph_t graph = nullptr;
-        svdag_status st = SVDAG_OK;
-        if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-            st = launch_phases(ctx, tool, cs);
-            const cudaError_t e = cudaStreamEndCapture(cs, &graph);
-            if (st == SVDAG_OK && e != cudaSuccess)
-                st = cuda_status(e);
-        } else {
-            st = SVDAG_ERR_CUDA;
-        }
-        if (st == SVDAG_OK && cudaGraphInstantiate(&ctx->graphs[g], graph, 0) != cudaSuccess)
-            st = SVDAG_ERR_CUDA;
-        if (graph)
-            cudaGraphDestroy(graph);
-        cudaStreamDestroy(cs);
-        if (st != SVDAG_OK) {
-            ctx->graphs[g] = nullptr;
-            return st;
-        }
+    switch (ed.tool) {
+    case SVDAG_TOOL_SPHERE_ADD:
+        return launch_edit<SVDAG_TOOL_SPHERE_ADD>(ctx, ed, record, s);
+    case SVDAG_TOOL_SPHERE_REMOVE:
+        return launch_edit<SVDAG_TOOL_SPHERE_REMOVE>(ctx, ed, record, s);
+    case SVDAG_TOOL_BOX_ADD:
+        return launch_edit<SVDAG_TOOL_BOX_ADD>(ctx, ed, record, s);
+    case SVDAG_TOOL_BOX_REMOVE:
+        return launch_edit<SVDAG_TOOL_BOX_REMOVE>(ctx, ed, record, s);
+    case SVDAG_TOOL_SPHERE_PAINT:
+        return launch_edit<SVDAG_TOOL_SPHERE_PAINT>(ctx, ed, record, s);
+    case SVDAG_TOOL_COPY:
+        return launch_edit<SVDAG_TOOL_COPY>(ctx, ed, record, s);
+    case SVDAG_TOOL_BOX_PAINT_NOISE:
+        return launch_edit<SVDAG_TOOL_BOX_PAINT_NOISE>(ctx, ed, record, s);
+    case SVDAG_TOOL_SPHERE_ERODE:
+        return launch_edit<SVDAG_TOOL_SPHERE_ERODE>(ctx, ed, record, s);
+    case kToolTerrain:
+        return launch_edit<kToolTerrain>(ctx, ed, record, s);
+    default:
+        return SVDAG_ERR_INVALID;
     }
-    SVDAG_CUDA(cudaGraphLaunch(ctx->graphs[g], s));
-    return SVDAG_OK;
-}
-
-// One editor: copied into the queue slot from host memory, then its phases.
-svdag_status launch_pipeline(svdag_ctx* ctx, const DevEditor& ed, cudaStream_t s, EditRecord* record, bool graphOk)
-{
-    EditQueue h {};
-    h.eds = nullptr;
-    h.slot = ed;
-    h.slot.record = record;
-    SVDAG_CUDA(cudaMemcpyAsync(ctx->queue, &h, sizeof(h), cudaMemcpyHostToDevice, s));
-    return run_phases(ctx, ed.tool, s, graphOk);
 }
 
 // Upper estimate of the leaves of an editor's intermediate SVO: the bounding volume in 4^3 bricks or,
@@ -1792,12 +2203,17 @@ bool subtree_node(const svdag_ctx* ctx, const DevEditor& e, uint32_t& level, uin
 
 constexpr unsigned long long kSubtreeScratch = 16ull << 20; // scratch slice of one subtree edit
 
-// Launches expanded editors with their editors and records in `region`. Large edits run as one launch
-// per phase at full occupancy. Runs of small edits are cut into groups of subtree edits whose nodes
-// are pairwise disjoint (one block per edit builds its subtree, then the paths from the root to the
-// subtrees are rebuilt and committed in order: k_edit_subtrees, k_edit_spines)
-// and the edits between them, which run one after another in
-// one persistent launch (block barriers are cheaper than launches for small SVOs).
+// Launches expanded editors with their editors and records in `region`: an edit as its chain of
+// launches, or a run of small edits whose nodes are pairwise disjoint as one group (one block per edit
+// builds its subtree, then the paths from the root to the subtrees are rebuilt and committed in order:
+// k_edit_subtrees, k_edit_spines), where that is the faster of the two. Measured for spheres and boxes
+// at depth 14: a chain takes 55 us and 5 us more per 1000 estimated leaves (radius 9: 68, radius 70: 113);
+// a group takes 60 us for its paths and its slowest block, which is 55 us and 35 us more per 1000
+// leaves (radius 20: 90, radius 70: 390-590). An edit alone in the one-block kernel is never faster than
+// its chain (radius 1: 57 against 55 us; radius 45: 200 against 98).
+double chain_us(double leaves) { return 55.0 + 0.005 * leaves; }
+double group_us(double mostLeaves) { return 60.0 + 55.0 + 0.035 * mostLeaves; }
+
 svdag_status launch_edits_at(svdag_ctx* ctx, const DevEditor* eds, uint32_t n, char* region, size_t regionBytes, cudaStream_t s)
 {
     const size_t edBytes = align256((size_t)n * sizeof(DevEditor));
@@ -1807,7 +2223,7 @@ svdag_status launch_edits_at(svdag_ctx* ctx, const DevEditor* eds, uint32_t n, c
     EditRecord* records = reinterpret_cast<EditRecord*>(region + edBytes);
     auto small = [&](uint32_t k) { return ctx->persistentLeaves > 0 && estimate_leaves(eds[k]) <= ctx->persistentLeaves; };
     // plan: [begin, end) segments of one kind each
-    enum Kind { LARGE, SEQUENTIAL, GROUP };
+    enum Kind { CHAINS, GROUP };
     struct Seg {
         uint32_t begin, end;
         Kind kind;
@@ -1825,7 +2241,7 @@ svdag_status launch_edits_at(svdag_ctx* ctx, const DevEditor* eds, uint32_t n, c
     };
     for (uint32_t k = 0; k < n;) {
         if (!small(k)) {
-            extend(k++, LARGE);
+            extend(k++, CHAINS);
             continue;
         }
         uint32_t e = k, lv[kMaxGroup], pt[kMaxGroup][3];
@@ -1840,9 +2256,20 @@ svdag_status launch_edits_at(svdag_ctx* ctx, const DevEditor* eds, uint32_t n, c
                 break;
             ++e;
         }
-        const uint32_t m = e - k;
+        // the prefix of the run that gains most as a group
+        uint32_t m = 0;
+        double chains = 0, most = 0, best = 0;
+        for (uint32_t q = k; q < e; ++q) {
+            const double leaves = estimate_leaves(eds[q]);
+            chains += chain_us(leaves);
+            most = std::max(most, leaves);
+            if (chains - group_us(most) > best) {
+                best = chains - group_us(most);
+                m = q + 1 - k;
+            }
+        }
         if (m < 2) {
-            extend(k++, SEQUENTIAL);
+            extend(k++, CHAINS);
             continue;
         }
         uint32_t* results = reinterpret_cast<uint32_t*>(ctx->scratch + align256((size_t)m * sizeof(EditCounters)));
@@ -1854,23 +2281,17 @@ svdag_status launch_edits_at(svdag_ctx* ctx, const DevEditor* eds, uint32_t n, c
                 ed.startPath[a] = pt[q][a];
             ed.tileOut = results + q;
         }
-        segs.push_back(Seg { k, e, GROUP });
-        k = e;
+        segs.push_back(Seg { k, k + m, GROUP });
+        k += m;
     }
     // a pageable source is staged before the call returns, so the vector may go
     SVDAG_CUDA(cudaMemcpyAsync(region, withRecords.data(), (size_t)n * sizeof(DevEditor), cudaMemcpyHostToDevice, s));
     const DevDag d = ctx->dag();
     for (const Seg& g : segs) {
         const uint32_t m = g.end - g.begin;
-        if (g.kind == LARGE) { // a run of editors through the queue: the first phase takes eds[cursor]
-            const EditQueue head { devEds + g.begin, 0, 0, {} };
-            SVDAG_CUDA(cudaMemcpyAsync(ctx->queue, &head, offsetof(EditQueue, slot), cudaMemcpyHostToDevice, s));
+        if (g.kind == CHAINS) {
             for (uint32_t k = g.begin; k < g.end; ++k)
-                SVDAG_TRY(run_phases(ctx, eds[k].tool, s, true));
-        } else if (g.kind == SEQUENTIAL) {
-            k_edit_block<<<1, kBlockThreads, 0, s>>>(d, eds[g.begin], devEds + g.begin, m, ctx->scratch, ctx->scratchBytes,
-                records + g.begin);
-            SVDAG_CUDA(cudaGetLastError());
+                SVDAG_TRY(launch_pipeline(ctx, eds[k], s, records + k));
         } else {
             // scratch: the group's counters, its result handles, the bucket locks, then one slice per edit
             const size_t cntBytes = align256((size_t)m * sizeof(EditCounters));
@@ -1938,7 +2359,7 @@ svdag_status run_edit(svdag_ctx* ctx, const svdag_edit* e, cudaStream_t s)
         if (ctx->persistentLeaves > 0 && estimate_leaves(eds[i]) <= ctx->persistentLeaves)
             SVDAG_TRY(launch_single_fused(ctx, eds[i], s));
         else
-            SVDAG_TRY(launch_pipeline(ctx, eds[i], s, nullptr, true));
+            SVDAG_TRY(launch_pipeline(ctx, eds[i], s, nullptr));
     }
     return SVDAG_OK;
 }
@@ -1989,14 +2410,13 @@ svdag_status build_scene_untiled(svdag_ctx* ctx, const DevEditor& ed, cudaStream
 {
     SVDAG_TRY(reset_dag(ctx, s));
     const DevDag d = ctx->dag();
-    {
-        EditQueue h {};
-        h.slot = ed;
-        SVDAG_CUDA(cudaMemcpyAsync(ctx->queue, &h, sizeof(h), cudaMemcpyHostToDevice, s));
-    }
-    k_edit_begin<<<1, 32, 0, s>>>(d, ctx->queue, ctx->scratch);
-    SVDAG_TRY(launch_build_any(ctx, kToolTerrain, s));
     const uint32_t LL = d.leafLevel;
+    SVDAG_TRY(launch_chained(k_edit_top<kToolTerrain>, 1, kBlockThreads, false, s, d, ed, ed.startLevel, ctx->scratch, ctx->scratchBytes));
+    for (uint32_t level = 0; level < LL; ++level)
+        SVDAG_TRY(launch_chained(k_build_level<kToolTerrain>, grid_for(ctx, level_bound(level) * 8, 256), 256, true, s, d, ed, level, ctx->scratch,
+            ctx->scratchBytes));
+    SVDAG_TRY(launch_chained(k_build_leaves<kToolTerrain>, grid_for(ctx, level_bound(LL) * 32, 256), 256, true, s, d, ed, ctx->scratch,
+        ctx->scratchBytes));
     for (int level = (int)LL; level >= 0; --level) {
         if (level < (int)LL)
             k_fix_level<<<grid_for(ctx, level_bound(level), 256), 256, 0, s>>>(d, level, 1, ctx->scratch);
@@ -2021,8 +2441,8 @@ svdag_status build_scene_untiled(svdag_ctx* ctx, const DevEditor& ed, cudaStream
         SVDAG_TRY(insert_canonical(ctx, (uint32_t)level, s));
         SVDAG_TRY(launch_insert(ctx, level, level_bound(level), s));
     }
-    k_edit_end<<<1, 32, 0, s>>>(d, ctx->scratch, ctx->queue);
-    SVDAG_CUDA(cudaGetLastError());
+    SVDAG_TRY(launch_chained(k_edit_bottom, 1, kBlockThreads, true, s, d, ed.startLevel, ed.startLevel, ed.builder, ed.tileOut, (EditRecord*)nullptr,
+        ctx->scratch));
     return read_status(ctx, s);
 }
 
@@ -2031,7 +2451,7 @@ svdag_status build_scene_untiled(svdag_ctx* ctx, const DevEditor& ed, cudaStream
 svdag_status launch_scene_tiles(svdag_ctx* ctx, const DevEditor* eds, uint32_t n, cudaStream_t s)
 {
     for (uint32_t i = 0; i < n; ++i) // tiles are large: one launch per phase at full occupancy
-        SVDAG_TRY(launch_pipeline(ctx, eds[i], s, nullptr, false));
+        SVDAG_TRY(launch_pipeline(ctx, eds[i], s, nullptr));
     return SVDAG_OK;
 }
 

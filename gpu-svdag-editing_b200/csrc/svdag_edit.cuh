@@ -14,7 +14,6 @@ enum : uint32_t { OP_SUBDIVIDE = 0, OP_FILL = 1, OP_EMPTY = 2, OP_KEEP = 3 };
 enum : uint32_t { ST_PARTIAL = 0, ST_FILLED = 1, ST_EMPTY = 2 };
 constexpr uint32_t kToolTerrain = 100; // internal: the procedural scene builder
 constexpr uint32_t kEmptyRep = 0xFFFFFFFEu; // dedup result of an empty SVO item
-constexpr int kNumGraphs = 10; // CUDA graphs of the phase launches: one per tool, the last for the scene builder
 
 struct EditRecord;
 
@@ -49,16 +48,6 @@ constexpr uint32_t kKeep = 0xFFFFFFFDu; // subtree edit: nothing committed
 struct EditRecord {
     uint32_t rootBefore, rootAfter, status, pad;
     unsigned long long edited, added, unique, svoItems;
-};
-
-// Editor of the running edit for the one-launch-per-phase form (and its CUDA graphs): the phase
-// kernels read `slot`; with `eds` set, the first phase copies eds[cursor] into the slot and the
-// last one advances the cursor, so one captured graph per tool serves every edit of a batch.
-struct EditQueue {
-    const DevEditor* eds;
-    uint32_t cursor;
-    uint32_t pad;
-    DevEditor slot;
 };
 
 struct WorkItem { // CreateIntermediateWorkItem (create_edit_svo.cu:55-65)

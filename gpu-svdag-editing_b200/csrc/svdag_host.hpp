@@ -27,8 +27,6 @@ struct svdag_ctx {
     unsigned long long scratchBytes = 0;
     char* batch = nullptr; // editors and per-edit records of a persistent batch launch
     unsigned long long batchBytes = 0;
-    svdag::EditQueue* queue = nullptr; // editor slot of the one-launch-per-phase form (end of the batch region)
-    cudaGraphExec_t graphs[svdag::kNumGraphs] = {}; // per tool: the phase launches of one edit
     uint32_t lastBatch = 0;
     uint32_t* items = nullptr; // item region
     unsigned long long itemWords = 0;
@@ -113,7 +111,7 @@ bool valid_edit(const svdag_edit* e);
 int expand_edit(const svdag_ctx* ctx, const svdag_edit& e, DevEditor* out);
 double estimate_leaves(const DevEditor& e);
 svdag_status launch_single_fused(svdag_ctx* ctx, const DevEditor& ed, cudaStream_t s);
-svdag_status launch_pipeline(svdag_ctx* ctx, const DevEditor& ed, cudaStream_t s, EditRecord* record, bool graphOk);
+svdag_status launch_pipeline(svdag_ctx* ctx, const DevEditor& ed, cudaStream_t s, EditRecord* record);
 // The batched table operations of the public API, by lane count (svdag_tables.cu).
 svdag_status table_add_lanes(svdag_table* t, const uint32_t* keys, const uint32_t* offsets, uint32_t n, unsigned long long totalWords,
     uint32_t* out, uint32_t lanes, cudaStream_t s);

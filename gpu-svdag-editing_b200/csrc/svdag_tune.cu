@@ -150,7 +150,7 @@ svdag_status tune_edits(svdag_ctx* ctx, const svdag_edit* edits, uint32_t n, svd
                 ++b;
             Timer& t = timers[used];
             cudaEventRecord(t.a, s);
-            SVDAG_TRY(form ? launch_single_fused(ctx, eds[j], s) : launch_pipeline(ctx, eds[j], s, nullptr, true));
+            SVDAG_TRY(form ? launch_single_fused(ctx, eds[j], s) : launch_pipeline(ctx, eds[j], s, nullptr));
             cudaEventRecord(t.b, s);
             const uint32_t tool = eds[j].tool < SVDAG_NUM_TOOLS ? eds[j].tool : 0u;
             bucketOf[used] = seen[form][tool] ? b : -1;

@@ -54,12 +54,12 @@ typedef enum svdag_status {
  * 2 + ceil(4 * popcount(64-bit voxel mask) / 32). Keys are self-describing. */
 typedef enum svdag_item_kind { SVDAG_KIND_NODE = 0, SVDAG_KIND_LEAF = 1 } svdag_item_kind;
 
-/* Launch every edit phase directly instead of replaying the tool's captured CUDA graph of the phase
- * launches (for profiling single phases). */
+/* Run every level's phases as launches of their own instead of the narrow levels (few items) of an edit
+ * together in one block (for profiling single phases). */
 #define SVDAG_FLAG_PHASE_KERNELS 1u
-/* Run edits whose intermediate SVO is estimated small (up to 16384 leaves) in the persistent kernel
- * (one CTA, block barriers between phases; a run of such edits is one launch) instead of the tool's
- * CUDA graph of the phase launches. svdag_autotune chooses the threshold by measurement. */
+/* Run single edits whose intermediate SVO is estimated small (up to 16384 leaves) in the persistent kernel
+ * (one CTA, block barriers between phases, one launch) instead of the chain of phase launches, and let
+ * batches group such edits. svdag_autotune chooses the threshold by measurement. */
 #define SVDAG_FLAG_PERSISTENT 2u
 
 typedef struct svdag_config {
@@ -172,8 +172,7 @@ svdag_status svdag_edit_apply(svdag_ctx* ctx, const svdag_edit* edit, void* stre
 /* Batched form: applies the edits in order with no host round trip between them, all reading their
  * editors from device memory. Consecutive small sphere/box add, remove and paint edits whose
  * footprints lie in pairwise disjoint subtrees are built side by side (one block each) and committed
- * in order; other small edits run one after another in one persistent launch; the others are
- * replayed through the tool's CUDA graph. The result, the undo frames and the records equal applying
+ * in order; the others run as a chain of launches each. The result, the undo frames and the records equal applying
  * the edits one by one. Each edit gets an svdag_edit_record. A move counts as two records (removal,
  * then paste). */
 svdag_status svdag_edit_apply_many(svdag_ctx* ctx, const svdag_edit* edits, uint32_t count, void* stream);
