@@ -75,6 +75,7 @@ struct EditCounters {
     uint32_t ffRan[kMaxLevels]; // discovery ran at this level
     uint32_t repCount[kMaxLevels]; // items left after intra-level dedup
     uint32_t repPerClass[kMaxLevels][kNumClasses];
+    uint32_t fullSeen[kMaxLevels]; // materials of the fully filled items counted in repCount
     unsigned long long oldRead, added, edited;
     unsigned long long offW[kMaxLevels]; // scratch byte offset of each level's work items
     unsigned long long offN[kMaxLevels]; // scratch byte offset of each level's SVO items

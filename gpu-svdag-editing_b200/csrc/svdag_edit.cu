@@ -946,12 +946,14 @@ __device__ __forceinline__ uint32_t dedup_item(unsigned long long* table, uint32
         }
         if ((uint32_t)(e >> 32) == hb) {
             const uint32_t j = (uint32_t)e - 1u;
-            const uint32_t* q = items + (size_t)j * kItemStride;
+            const uint2* q = reinterpret_cast<const uint2*>(items + (size_t)j * kItemStride);
             bool same = true;
 #pragma unroll
-            for (uint32_t k = 0; k < kItemStride; ++k)
-                if (k < nw)
-                    same &= __ldcg(q + k) == w[k];
+            for (uint32_t k = 0; k < kItemStride; k += 2) // items are padded with zeros to ten words, w is not
+                if (k < nw) {
+                    const uint2 v = __ldcg(q + k / 2);
+                    same &= v.x == w[k] && (k + 1 >= nw || v.y == w[k + 1]);
+                }
             if (same)
                 return j;
         }
@@ -1091,37 +1093,89 @@ __device__ void ph_merge_level(const DevDag& d, uint32_t level, char* scratch)
     uint32_t* items = reinterpret_cast<uint32_t*>(scratch + E.offN[level]);
     const DevTable& t = d.ctl->tables[level]; // in memory: a copy indexed by size class would live on the stack
     Grp<1> g;
+    const uint32_t lane = threadIdx.x & 31u;
     uint32_t full = 0, reps = 0, added = 0;
-    for (uint32_t i = ph_block(d) * blockDim.x + threadIdx.x; i < n; i += ph_grid(d) * blockDim.x) {
-        uint32_t* it = items + (size_t)i * kItemStride;
+    for (uint32_t base = ph_block(d) * blockDim.x; base < n; base += ph_grid(d) * blockDim.x) { // whole warps
+        const uint32_t i = base + threadIdx.x;
+        uint2* it = reinterpret_cast<uint2*>(items + (size_t)i * kItemStride);
         Key<1> key;
 #pragma unroll
-        for (uint32_t j = 0; j < kItemStride; ++j)
-            key.w[j] = it[j];
-        if (!isLeaf) {
-            full += fix_node(d, level, gate, ArrayChildren { repC, hC }, key.w) ? 1u : 0u;
+        for (uint32_t j = 0; j < kItemStride; j += 2) {
+            const uint2 v = i < n ? it[j / 2] : make_uint2(0, 0);
+            key.w[j] = v.x;
+            key.w[j + 1] = v.y;
+        }
+        // A fully filled item of one material is the level's canonical one, whose handle is known: the
+        // interior of a solid needs no search (every thread of it would read the same few entries).
+        uint32_t canonical = kNone;
+        if (isLeaf) {
+            if ((key.w[0] & key.w[1]) == 0xFFFFFFFFu) {
+                const uint32_t m = key.w[2] & 0xFu;
+                bool same = key.w[2] == m * 0x11111111u;
 #pragma unroll
-            for (uint32_t j = 0; j < kItemStride; ++j)
-                it[j] = key.w[j];
+                for (uint32_t j = 3; j < kItemStride; ++j)
+                    same = same && key.w[j] == key.w[2];
+                canonical = same ? m : kNone;
+            }
+        } else if (i < n) {
+            if (fix_node(d, level, gate, ArrayChildren { repC, hC }, key.w)) {
+                ++full;
+                const uint32_t m = (key.w[0] >> 9) & 0xFu, below = d.ctl->fullyFilled[level + 1][m];
+                bool same = true;
+#pragma unroll
+                for (uint32_t j = 1; j < 9; ++j)
+                    same = same && key.w[j] == below;
+                canonical = same ? m : kNone;
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < kItemStride; j += 2)
+                it[j / 2] = make_uint2(key.w[j], key.w[j + 1]);
             if (n > 1)
                 fence_release(); // the content is visible before the dedup entry that points at it
         }
         const bool isEmpty = isLeaf ? (key.w[0] == 0 && key.w[1] == 0) : ((key.w[0] & 0xFFu) == 0);
-        if (isEmpty) {
+        if (canonical != kNone) { // its own representative, counted once a level and material
+            rep[i] = i;
+            handle[i] = d.ctl->fullyFilled[level][canonical];
+            const uint32_t bit = 1u << canonical;
+            if (!(__ldcg(&E.fullSeen[level]) & bit) && !(atomicOr(&E.fullSeen[level], bit) & bit))
+                ++reps;
+        } else if (i < n && isEmpty) {
             rep[i] = kEmptyRep;
-            continue;
         }
+        const bool pending = i < n && !isEmpty && canonical == kNone;
         key.n = isLeaf ? dev_leaf_words(key.w[0], key.w[1]) : dev_node_words(key.w[0]);
         hash_words(key.w, key.n, key.ha, key.hb);
-        // a level of one item has no duplicates (the top levels of a small edit)
-        const uint32_t r = n > 1 ? dedup_item(table, m.cap - 1u, items, i, key.w, key.n, key.ha, key.hb) : i;
-        rep[i] = r;
-        if (r != i)
-            continue;
-        ++reps;
-        bool ins = false;
-        handle[i] = table_find_or_insert<1, SHARED ? kInsertShared : kInsertLaunch>(g, d, t, key, ins);
-        added += ins ? 1u : 0u;
+        // Equal items of a warp (repetitive regions) take one search between them.
+        uint32_t lead = lane;
+        if (n > 1) {
+            const uint32_t live = __ballot_sync(0xFFFFFFFFu, pending);
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key.ha) & live;
+            const uint32_t first = pending ? (uint32_t)__ffs(peers) - 1u : lane;
+            if (__any_sync(0xFFFFFFFFu, first != lane)) {
+                bool same = true;
+#pragma unroll
+                for (uint32_t j = 0; j < kItemStride; ++j) {
+                    const uint32_t mine = j < key.n ? key.w[j] : 0u;
+                    same &= __shfl_sync(0xFFFFFFFFu, mine, first) == mine;
+                }
+                lead = same ? first : lane;
+            }
+        }
+        uint32_t r = i;
+        if (pending && lead == lane) {
+            // a level of one item has no duplicates (the top levels of a small edit)
+            r = n > 1 ? dedup_item(table, m.cap - 1u, items, i, key.w, key.n, key.ha, key.hb) : i;
+            if (r == i) {
+                ++reps;
+                bool ins = false;
+                handle[i] = table_find_or_insert<1, SHARED ? kInsertShared : kInsertLaunch>(g, d, t, key, ins);
+                added += ins ? 1u : 0u;
+            }
+        }
+        r = __shfl_sync(0xFFFFFFFFu, r, lead);
+        if (pending)
+            rep[i] = r;
     }
     if (full)
         atomicAdd(&E.ffCount[level], full);
