@@ -157,7 +157,10 @@ __device__ __forceinline__ uint32_t should_edit(const DevEditor& e, uint32_t px,
 // Terms of the overlap tests for one voxel coordinate v of axis a (depth 0): the tests of box_overlap
 // and sphere_overlap are per axis, combined in axis order, so a leaf's voxels share them. A sphere's
 // term is what its distance test subtracts on that axis (0 where it subtracts nothing, which leaves the
-// running value as it is).
+// running value as it is). In the leaf phase the overlap test alone decides a voxel: Keep when it does
+// not overlap, Empty for the painting and erosion tools on an empty voxel, else get_new_value, in which
+// Fill and Subdivide of a voxel end alike (the fill material, nothing, or the paint material), and a
+// voxel that is contained also overlaps.
 __device__ __forceinline__ float coord_float(uint32_t v) // float(v) for v < 2^23, by the exponent instead of a conversion
 {
     return __uint_as_float(0x4B000000u + v) - 8388608.0f;
@@ -178,31 +181,6 @@ __device__ __forceinline__ AxisTerm axis_term(const DevEditor& e, int a, uint32_
     else if (e.center[a] > nmax)
         t.dist = sqf(e.center[a] - nmax);
     return t;
-}
-
-// should_edit for one voxel (depth 0) in the leaf phase, from its axis terms. For the sphere and box
-// add/remove tools and the sphere paint, Fill and Subdivide of a voxel end in the same get_new_value
-// (the fill material, nothing, or the paint material), and a node that is contained also overlaps, so
-// the overlap test alone decides the voxel: Keep when it does not overlap, Empty for the painting and
-// erosion tools on an empty voxel, else Subdivide.
-template <uint32_t TOOL>
-__device__ __forceinline__ uint32_t voxel_op(const DevEditor& e, const AxisTerm& x, const AxisTerm& y, const AxisTerm& z, bool filled)
-{
-    bool overlaps;
-    if constexpr (TOOL == SVDAG_TOOL_BOX_ADD || TOOL == SVDAG_TOOL_BOX_REMOVE || TOOL == SVDAG_TOOL_BOX_PAINT_NOISE || TOOL == SVDAG_TOOL_COPY) {
-        overlaps = x.meets && y.meets && z.meets;
-    } else {
-        float dist = e.radiusSquared;
-        dist -= x.dist;
-        dist -= y.dist;
-        dist -= z.dist;
-        overlaps = dist > 0;
-    }
-    if (!overlaps)
-        return OP_KEEP;
-    if ((TOOL == SVDAG_TOOL_SPHERE_PAINT || TOOL == SVDAG_TOOL_BOX_PAINT_NOISE || TOOL == SVDAG_TOOL_SPHERE_ERODE) && !filled)
-        return OP_EMPTY;
-    return OP_SUBDIVIDE;
 }
 
 // MyGpuCopyEditor::should_edit with state (the "#if 1" form, my_gpu_dag_editors.h:173-217): the children of
@@ -440,23 +418,57 @@ __device__ void ph_build_level(const DevDag& d, const DevEditor& e, uint32_t lev
     }
 }
 
-// One warp per leaf (createIntermediateSvoStructure_leaf_workgroup, create_edit_svo.cu:321-426, which uses
-// a 64-thread block per leaf). A voxel's index in the leaf's mask is the bits (x1 y1 z1 x0 y0 z0) of its
-// coordinates; lane l = (x1 y1 x0 y0 z0) owns the two voxels with z1 = 0 and 1, so they share their x
-// and y terms and the lerps along x and y. The ballots of the two give the mask by interleaving their
-// bytes. Bound by the integer pipes: population counts (16 a clock an SM), shuffles and multiplies; so
-// old materials are looked up only where a voxel keeps one, and a leaf that comes out full or empty
-// skips the ranks and the packing through shared memory.
-// Measured against lanes owning voxels l and l + 32 with every lookup done for every leaf: 1024^3 noise paint
-// 6.2 -> 3.8 ms, sphere removal of radius 1024 246 -> 181 us, erosion of radius 40 32 -> 20 us.
-__device__ __forceinline__ uint32_t leaf_mask_lo(uint32_t b0, uint32_t b1) { return __byte_perm(b0, b1, 0x5140); }
-__device__ __forceinline__ uint32_t leaf_mask_hi(uint32_t b0, uint32_t b1) { return __byte_perm(b0, b1, 0x7362); }
+// Eight lanes per leaf, four leaves a warp (createIntermediateSvoStructure_leaf_workgroup,
+// create_edit_svo.cu:321-426, uses a 64-thread block per leaf). A voxel's index in the leaf's mask is the
+// bits (x1 y1 z1 x0 y0 z0) of its coordinates, so lane q = (x1 y1 z1) owns mask byte q: a 2^3 block, whose
+// tests and lerps share their axis terms, whose old materials are consecutive nibbles, and whose new
+// materials are material word q when the leaf comes out full. Otherwise each lane's nibbles go to their
+// place among the words by shuffles. Bound by the integer pipes; what a leaf needs once (loads,
+// addresses, lattice corners) costs a quarter of a warp instruction. Work items are loaded three leaves
+// ahead, old masks two, old materials one.
+// Measured against a warp per leaf with two voxels a lane: 1024^3 noise paint 3.97 -> 1.75 ms, 512^3 copy 466 ->
+// 218 us, a tile of a depth-13 terrain 4.7 -> 1.1 ms.
 template <uint32_t TOOL>
-__device__ void ph_build_leaves(const DevDag& d, const DevEditor& e, char* scratch, unsigned long long scratchBytes)
+constexpr uint32_t leaf_shared_words() // shared words of a leaf's eight lanes: source leaves (copy), neighbour masks (erosion)
 {
-    __shared__ __align__(16) uint32_t packBuf[16][16]; // per warp of a block of up to 512 threads: 64 material bytes
-    __shared__ uint2 erodeBuf[TOOL == SVDAG_TOOL_SPHERE_ERODE ? 16 : 1][27]; // erosion: per warp, the neighbour leaf masks
-    __shared__ __align__(16) uint32_t copyBuf[TOOL == SVDAG_TOOL_COPY ? 16 : 1][8][12]; // copy: per warp, the source leaves
+    return TOOL == SVDAG_TOOL_COPY ? 8u * 12u : TOOL == SVDAG_TOOL_SPHERE_ERODE ? 27u * 2u : 1u;
+}
+
+// Heights of a lane's two columns (x0, z) and (x0 + 1, z) of a leaf. A leaf lies in one lattice cell of every
+// octave whose cells are 4 voxels or larger, so the eight lanes of a leaf compute the corner values of all
+// octaves together (four corners an octave, two octaves a round) and each interpolates its own columns.
+__device__ __forceinline__ void leaf_heights(const SceneParams& p, uint32_t q, uint32_t x0, uint32_t z, uint32_t (&h)[2])
+{
+    uint32_t f[2] = { 0, 0 }; // at most 65535 (2^octaves - 1): fits for the 16 octaves allowed
+    const uint32_t octaves = p.terrain.octaves;
+    for (uint32_t o = 0; o < octaves; o += 2) {
+        const uint32_t mo = o + (q >> 2), mc = terrain_cell_log2(p, mo);
+        const uint32_t mine = terrain_lattice(p, (x0 >> mc) + ((q >> 1) & 1u), (z >> mc) + (q & 1u), mo);
+#pragma unroll
+        for (uint32_t k = 0; k < 2; ++k) {
+            uint32_t v[4]; // corners (x, z) = (0, 0), (0, 1), (1, 0), (1, 1)
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j)
+                v[j] = __shfl_sync(0xFFFFFFFFu, mine, 4u * k + j, 8);
+            if (o + k < octaves) {
+                const uint32_t c = terrain_cell_log2(p, o + k), up = octaves - 1u - (o + k);
+                const uint32_t sz = smooth16u(cell_fraction(z, c));
+#pragma unroll
+                for (uint32_t dx = 0; dx < 2; ++dx) {
+                    const uint32_t sx = smooth16u(cell_fraction(x0 + dx, c));
+                    const uint32_t a = lerp16u(v[0], v[2], sx, 2u * sx), b = lerp16u(v[1], v[3], sx, 2u * sx);
+                    f[dx] += lerp16u(a, b, sz, 2u * sz) << up;
+                }
+            }
+        }
+    }
+    h[0] = terrain_height_from_fbm(p, f[0]);
+    h[1] = terrain_height_from_fbm(p, f[1]);
+}
+
+template <uint32_t TOOL>
+__device__ void ph_build_leaves(const DevDag& d, const DevEditor& e, char* scratch, unsigned long long scratchBytes, uint32_t* shared)
+{
     EditCounters& E = *d.edit;
     const uint32_t LL = d.leafLevel;
     const unsigned long long stride = work_stride(TOOL);
@@ -506,274 +518,329 @@ __device__ void ph_build_leaves(const DevDag& d, const DevEditor& e, char* scrat
         }
     }
 
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t warpsTotal = ph_grid(d) * (blockDim.x >> 5);
+    constexpr bool kBox = TOOL == SVDAG_TOOL_BOX_ADD || TOOL == SVDAG_TOOL_BOX_REMOVE || TOOL == SVDAG_TOOL_BOX_PAINT_NOISE || TOOL == SVDAG_TOOL_COPY;
+    const uint32_t lane = threadIdx.x & 31u, q = lane & 7u, byteAt = 8u * (q & 3u);
+    uint32_t* sh = shared + (threadIdx.x >> 3) * leaf_shared_words<TOOL>();
+    const uint32_t step = ph_grid(d) * (blockDim.x >> 5) * 4u;
     uint32_t edited = 0, oldRead = 0, fullLeaves = 0; // of this lane's leaves: far below 2^32
-    // Software pipeline over the warp's leaves: the work item two ahead and the old leaf one ahead are
-    // in flight while a leaf is computed (every valid handle has 16 readable words, so the ten words
-    // of a leaf are fetched at once and trimmed to its size afterwards).
     auto work_at = [&](uint32_t k) {
         return k < n ? *reinterpret_cast<const WorkItem*>(scratch + offW + k * stride) : WorkItem { 0, 0, 0, kNone };
     };
-    auto leaf_word = [&](uint32_t h) { return (h != kNone && lane < kItemStride) ? item_ptr(d, h)[lane] : 0u; };
-    uint32_t i = ph_block(d) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    WorkItem w = work_at(i), wn = work_at(i + warpsTotal);
-    uint32_t owRaw = leaf_word(w.handle);
-    for (; i < n; i += warpsTotal) {
-        const WorkItem wnn = work_at(i + 2 * warpsTotal);
-        const uint32_t owNext = leaf_word(wn.handle);
-        // old leaf words (lanes 0..9; a stored voxel's material lies within its words)
-        const uint32_t lo = __shfl_sync(0xFFFFFFFFu, owRaw, 0), hi = __shfl_sync(0xFFFFFFFFu, owRaw, 1);
-        if (w.handle != kNone && lane == 0)
-            ++oldRead;
-        uint32_t th = 0; // scene: terrain column heights in lanes 0..15
-        if constexpr (TOOL == kToolTerrain) {
-            if (lane < 16)
-                th = terrain_height(e.scene, (w.x << 2) + (lane >> 2), (w.z << 2) + (lane & 3u));
+    auto mask_of = [&](uint32_t h) { // the old leaf's mask words (every valid handle has 16 readable words)
+        if (TOOL == kToolTerrain || h == kNone)
+            return make_uint2(0, 0);
+        return *reinterpret_cast<const uint2*>(item_ptr(d, h));
+    };
+    auto below = [&](uint2 m) { // set voxels before this lane's byte
+        const uint32_t under = (1u << byteAt) - 1u;
+        return q < 4u ? (uint32_t)__popc(m.x & under) : (uint32_t)(__popc(m.x) + __popc(m.y & under));
+    };
+    struct Old {
+        uint32_t a, b, shift; // the words with this lane's old materials, from nibble shift / 4 of `a` on
+    };
+    auto materials_of = [&](uint32_t h, uint2 m) {
+        Old o { 0, 0, 0 };
+        if (TOOL != kToolTerrain && h != kNone) {
+            const uint32_t at = below(m);
+            const uint32_t* p = item_ptr(d, h) + 2u + (at >> 3);
+            o = Old { p[0], p[1], 4u * (at & 7u) };
         }
-        uint32_t corners[8] = {}; // noise paint: lattice corners of the leaf's cell, one per lane 0..7
-        if constexpr (TOOL == SVDAG_TOOL_BOX_PAINT_NOISE) {
-            if (e.noiseCellLog2 >= 2) {
-                const uint32_t cl = e.noiseCellLog2;
-                const uint32_t mine = lattice3(e.noiseSeed, ((w.x << 2) >> cl) + ((lane >> 2) & 1u), ((w.y << 2) >> cl) + ((lane >> 1) & 1u),
-                    ((w.z << 2) >> cl) + (lane & 1u));
+        return o;
+    };
+    uint32_t i = (ph_block(d) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 4u + (lane >> 3);
+    WorkItem w = work_at(i), w1 = work_at(i + step), w2 = work_at(i + 2u * step);
+    uint2 om = mask_of(w.handle), om1 = mask_of(w1.handle);
+    Old old = materials_of(w.handle, om);
+    for (uint32_t base = i - (lane >> 3); base < n; base += step, i += step) { // whole warps
+        const WorkItem w3 = work_at(i + 3u * step);
+        const uint2 om2 = mask_of(w2.handle);
+        const Old old1 = materials_of(w1.handle, om1);
+        const bool active = i < n;
+        if (TOOL != kToolTerrain && w.handle != kNone && q == 0)
+            ++oldRead;
+        const uint32_t obyte = ((q < 4u ? om.x : om.y) >> byteAt) & 0xFFu;
+        const uint32_t vx = (w.x << 2) | ((q >> 1) & 2u), vy = (w.y << 2) | (q & 2u), vz = (w.z << 2) | ((q << 1) & 2u);
+        // bits of voxel j = (dx dy dz) of the block that the edit does not keep
+        uint32_t meets = 0;
+        if constexpr (TOOL != kToolTerrain) {
+            AxisTerm ax[2], ay[2], az[2];
+#pragma unroll
+            for (uint32_t k = 0; k < 2; ++k) {
+                ax[k] = axis_term<TOOL>(e, 0, vx + k);
+                ay[k] = axis_term<TOOL>(e, 1, vy + k);
+                az[k] = axis_term<TOOL>(e, 2, vz + k);
+            }
+            if constexpr (kBox) {
+                meets = ((ax[0].meets ? 0x0Fu : 0u) | (ax[1].meets ? 0xF0u : 0u)) & ((ay[0].meets ? 0x33u : 0u) | (ay[1].meets ? 0xCCu : 0u))
+                    & ((az[0].meets ? 0x55u : 0u) | (az[1].meets ? 0xAAu : 0u));
+            } else { // sphere_overlap: the squared radius less the axis terms in axis order, still positive
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j) {
+                    float dist = e.radiusSquared;
+                    dist -= ax[j >> 2].dist;
+                    dist -= ay[(j >> 1) & 1u].dist;
+                    dist -= az[j & 1u].dist;
+                    meets |= dist > 0 ? 1u << j : 0u;
+                }
+            }
+            if (!active)
+                meets = 0;
+            edited += (uint32_t)__popc(meets);
+        } else if (active) {
+            edited += 8u;
+        }
+
+        // New mask byte and the new materials: of every voxel in `mats` (nibble j) where the edit gives
+        // one, else the old ones.
+        uint32_t nbyte = obyte, given = 0, mats = 0;
+        if constexpr (TOOL == kToolTerrain) {
+            uint32_t h[2]; // columns (vx, z) and (vx + 1, z): the lanes of the two halves in y take one z each
+            const uint32_t z = vz + ((q >> 1) & 1u);
+            if (terrain_cell_log2(e.scene, e.scene.terrain.octaves - 1u) >= 2u) {
+                leaf_heights(e.scene, q, vx, z, h);
+            } else {
+                h[0] = active ? terrain_height(e.scene, vx, z) : 0u;
+                h[1] = active ? terrain_height(e.scene, vx + 1u, z) : 0u;
+            }
+            const uint32_t g0 = __shfl_xor_sync(0xFFFFFFFFu, h[0], 2), g1 = __shfl_xor_sync(0xFFFFFFFFu, h[1], 2);
+            const uint32_t col[4] = { q & 2u ? g0 : h[0], q & 2u ? h[0] : g0, q & 2u ? g1 : h[1], q & 2u ? h[1] : g1 }; // (dx dz)
+            const uint32_t m0 = terrain_material(e.scene, vy), m1 = terrain_material(e.scene, vy + 1u);
+            nbyte = 0;
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) { // scene_voxel: below the surface, then the structures over it
+                const uint32_t dy = (j >> 1) & 1u;
+                nbyte |= vy + dy < col[(j >> 2) * 2u + (j & 1u)] ? 1u << j : 0u;
+                mats |= (dy ? m1 : m0) << (4u * j);
+            }
+            if (e.scene.numStructures && active) { // in increasing index order: the last one that contains a voxel stays
+                const uint32_t cell = (vz >> e.scene.cellLog2) * e.scene.cellsPerAxis + (vx >> e.scene.cellLog2);
+                for (uint32_t k = e.scene.cellStart[cell]; k < e.scene.cellStart[cell + 1]; ++k) {
+                    const Structure& st = e.scene.structures[e.scene.cellList[k]];
+                    if ((int32_t)vx + 1 < st.lo[0] || (int32_t)vx >= st.hi[0] || (int32_t)vy + 1 < st.lo[1] || (int32_t)vy >= st.hi[1]
+                        || (int32_t)vz + 1 < st.lo[2] || (int32_t)vz >= st.hi[2])
+                        continue;
+#pragma unroll
+                    for (uint32_t j = 0; j < 8; ++j)
+                        if (structure_contains(st, (int32_t)(vx + (j >> 2)), (int32_t)(vy + ((j >> 1) & 1u)), (int32_t)(vz + (j & 1u)))) {
+                            nbyte |= 1u << j;
+                            mats = (mats & ~(0xFu << (4u * j))) | (st.material << (4u * j));
+                        }
+                }
+            }
+            nbyte = active ? nbyte : 0u;
+            given = nbyte;
+        } else if constexpr (TOOL == SVDAG_TOOL_BOX_ADD || TOOL == SVDAG_TOOL_SPHERE_ADD) {
+            nbyte = obyte | meets;
+            given = meets;
+            mats = e.material * 0x11111111u;
+        } else if constexpr (TOOL == SVDAG_TOOL_BOX_REMOVE || TOOL == SVDAG_TOOL_SPHERE_REMOVE) {
+            nbyte = obyte & ~meets;
+        } else if constexpr (TOOL == SVDAG_TOOL_SPHERE_PAINT) {
+            given = meets;
+            mats = e.material * 0x11111111u;
+        } else if constexpr (TOOL == SVDAG_TOOL_BOX_PAINT_NOISE) {
+            given = meets & obyte;
+            const uint32_t cl = e.noiseCellLog2;
+            if (cl >= 2) { // a leaf lies in one lattice cell: its eight corners, one a lane
+                const uint32_t mine = lattice3(e.noiseSeed, (vx >> cl) + ((q >> 2) & 1u), (vy >> cl) + ((q >> 1) & 1u), (vz >> cl) + (q & 1u));
+                uint32_t corner[8];
 #pragma unroll
                 for (uint32_t k = 0; k < 8; ++k)
-                    corners[k] = __shfl_sync(0xFFFFFFFFu, mine, k);
-            }
-        }
-        // erosion: the 27 leaves around this one in the DAG before the edit (lane k: offset
-        // (k / 9, k / 3 % 3, k % 3) - 1, coordinates wrapping as the reference's unsigned paths do)
-        if constexpr (TOOL == SVDAG_TOOL_SPHERE_ERODE) {
-            uint32_t nlo = 0, nhi = 0;
-            if (lane < 27) {
-                const uint32_t lmask = (1u << LL) - 1u;
-                const uint32_t lx = (w.x + lane / 9u - 1u) & lmask, ly = (w.y + (lane / 3u) % 3u - 1u) & lmask, lz = (w.z + lane % 3u - 1u) & lmask;
-                uint32_t h = E.rootBefore;
-                for (uint32_t l = 0; l < LL && h != kNone; ++l) {
-                    const uint32_t s = LL - 1u - l;
-                    const uint32_t c = (((lx >> s) & 1u) << 2) | (((ly >> s) & 1u) << 1) | ((lz >> s) & 1u);
-                    const uint32_t* node = item_ptr(d, h);
-                    const uint32_t m = node[0] & 0xFFu;
-                    h = ((m >> c) & 1u) ? node[1 + __popc(m & ((1u << c) - 1u))] : kNone;
+                    corner[k] = __shfl_sync(0xFFFFFFFFu, mine, k, 8);
+#pragma unroll
+                for (uint32_t dx = 0; dx < 2; ++dx) { // lerps along x, then y, then z, as noise_material's
+                    const uint32_t sx = smooth16u(cell_fraction(vx + dx, cl));
+                    uint32_t lx[4];
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k)
+                        lx[k] = lerp16u(corner[k], corner[k + 4], sx, 2u * sx);
+#pragma unroll
+                    for (uint32_t dy = 0; dy < 2; ++dy) {
+                        const uint32_t sy = smooth16u(cell_fraction(vy + dy, cl));
+                        const uint32_t a = lerp16u(lx[0], lx[2], sy, 2u * sy), b = lerp16u(lx[1], lx[3], sy, 2u * sy);
+#pragma unroll
+                        for (uint32_t dz = 0; dz < 2; ++dz) {
+                            const uint32_t sz = smooth16u(cell_fraction(vz + dz, cl));
+                            mats |= ((lerp16u(a, b, sz, 2u * sz) >> 12) & 0xFu) << (4u * (dx * 4u + dy * 2u + dz));
+                        }
+                    }
                 }
-                if (h != kNone) {
-                    const uint32_t* lp = item_ptr(d, h);
-                    nlo = lp[0];
-                    nhi = lp[1];
+            } else {
+                for (uint32_t j = 0; j < 8; ++j)
+                    if ((given >> j) & 1u)
+                        mats |= noise_material(e.noiseSeed, cl, vx + (j >> 2), vy + ((j >> 1) & 1u), vz + (j & 1u)) << (4u * j);
+            }
+        } else if constexpr (TOOL == SVDAG_TOOL_SPHERE_ERODE) { // get_new_value, :564-588
+            // the 27 leaves around this one in the DAG before the edit (k: offset (k / 9, k / 3 % 3, k % 3) - 1,
+            // coordinates wrapping as the reference's unsigned paths do), four descents a lane side by side
+            uint2* nb = reinterpret_cast<uint2*>(sh);
+            uint32_t h[4], lx[4], ly[4], lz[4];
+            const uint32_t lmask = (1u << LL) - 1u;
+#pragma unroll
+            for (uint32_t r = 0; r < 4; ++r) {
+                const uint32_t k = q + 8u * r;
+                lx[r] = (w.x + k / 9u - 1u) & lmask;
+                ly[r] = (w.y + (k / 3u) % 3u - 1u) & lmask;
+                lz[r] = (w.z + k % 3u - 1u) & lmask;
+                h[r] = active && k < 27u ? E.rootBefore : kNone;
+            }
+            for (uint32_t l = 0; l < LL; ++l) {
+                const uint32_t s = LL - 1u - l;
+                uint32_t head[4];
+#pragma unroll
+                for (uint32_t r = 0; r < 4; ++r)
+                    head[r] = h[r] != kNone ? item_ptr(d, h[r])[0] & 0xFFu : 0u;
+#pragma unroll
+                for (uint32_t r = 0; r < 4; ++r) {
+                    const uint32_t c = (((lx[r] >> s) & 1u) << 2) | (((ly[r] >> s) & 1u) << 1) | ((lz[r] >> s) & 1u);
+                    h[r] = (head[r] >> c) & 1u ? item_ptr(d, h[r])[1 + __popc(head[r] & ((1u << c) - 1u))] : kNone;
                 }
             }
-            uint2* nb = erodeBuf[threadIdx.x >> 5];
             __syncwarp();
-            if (lane < 27)
-                nb[lane] = make_uint2(nlo, nhi);
+#pragma unroll
+            for (uint32_t r = 0; r < 4; ++r)
+                if (q + 8u * r < 27u)
+                    nb[q + 8u * r] = h[r] != kNone ? *reinterpret_cast<const uint2*>(item_ptr(d, h[r])) : make_uint2(0, 0);
             __syncwarp();
-        }
-        // copy: a leaf's source box meets at most two leaves an axis; they are fetched once, all words at a
-        // time, into the slot of their place in that 2 x 2 x 2 block (absent ones read as empty)
-        uint32_t base[3] = {};
-        if constexpr (TOOL == SVDAG_TOOL_COPY) {
+            const uint32_t tested = meets & obyte;
+            if (tested) { // filled voxels of the 4^3 block around this lane's, bit 16a + 4b + c
+                unsigned long long around = 0;
+                for (uint32_t a = 0; a < 4; ++a)
+                    for (uint32_t b = 0; b < 4; ++b) {
+                        const uint32_t qx = ((q >> 1) & 2u) + a + 3u, qy = (q & 2u) + b + 3u; // leaf coordinate + 4 (3 .. 8)
+                        const uint32_t xy = ((qx & 1u) ? 4u : 0u) | ((qy & 1u) ? 2u : 0u) | ((qx & 2u) ? 32u : 0u) | ((qy & 2u) ? 16u : 0u);
+                        const uint2* row = nb + (qx >> 2) * 9u + (qy >> 2) * 3u;
+#pragma unroll
+                        for (uint32_t c = 0; c < 4; ++c) {
+                            const uint32_t qz = ((q << 1) & 2u) + c + 3u;
+                            const uint32_t bit = xy | ((qz & 1u) ? 1u : 0u) | ((qz & 2u) ? 8u : 0u);
+                            const uint2 m = row[qz >> 2];
+                            around |= (unsigned long long)(((bit & 32u ? m.y : m.x) >> (bit & 31u)) & 1u) << (16u * a + 4u * b + c);
+                        }
+                    }
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j) {
+                    const unsigned long long cube = 0x0000077707770777ull << (16u * (j >> 2) + 4u * ((j >> 1) & 1u) + (j & 1u));
+                    // the voxel itself is filled: its 26 neighbours are one less
+                    if (((tested >> j) & 1u) && (uint32_t)__popcll(around & cube) - 1u <= e.noiseSeed)
+                        nbyte &= ~(1u << j);
+                }
+            }
+        } else if constexpr (TOOL == SVDAG_TOOL_COPY) { // get_new_value(uint3, optional, State), :225-252
+            // a leaf's source box meets at most two leaves an axis; lane q fetches the list's q-th source leaf
+            // into the slot of its place in that 2 x 2 x 2 block (absent ones read as empty)
             const uint32_t at[3] = { w.x << 2, w.y << 2, w.z << 2 };
+            uint32_t first[3];
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                const int first = (int)at[a] + e.iDestToSource[a];
-                base[a] = (uint32_t)(first > 0 ? first : 0) >> 2;
+                const int f = (int)at[a] + e.iDestToSource[a];
+                first[a] = (uint32_t)(f > 0 ? f : 0) >> 2;
             }
             CopyParent par { 0, 0, 0, kNone };
-            if (lane < 8)
-                par = reinterpret_cast<const CopyParent*>(scratch + offW + i * stride + 16)[lane];
-            const uint32_t ends = __ballot_sync(0xFFFFFFFFu, par.handle == kNone); // a list ends at its first kNone
-            const uint32_t rx = par.x - base[0], ry = par.y - base[1], rz = par.z - base[2];
-            uint32_t slot = (rx * 2u + ry) * 2u + rz;
-            if (lane + 1u >= (uint32_t)__ffs(ends) || rx > 1u || ry > 1u || rz > 1u)
-                slot = 8u;
-            uint32_t (*leaves)[12] = copyBuf[threadIdx.x >> 5];
-            __syncwarp();
-            if (lane < 8)
-                leaves[lane][0] = leaves[lane][1] = 0u;
-            __syncwarp();
-            uint32_t v[3], to[3];
-#pragma unroll
-            for (uint32_t r = 0; r < 3; ++r) {
-                const uint32_t k = lane + 32u * r, p = k / kItemStride;
-                const uint32_t hp = __shfl_sync(0xFFFFFFFFu, par.handle, p & 7u), sp = __shfl_sync(0xFFFFFFFFu, slot, p & 7u);
-                to[r] = p < 8u ? sp : 8u;
-                v[r] = to[r] < 8u ? item_ptr(d, hp)[k % kItemStride] : 0u;
+            if (active)
+                par = reinterpret_cast<const CopyParent*>(scratch + offW + i * stride + 16)[q];
+            const uint32_t ends = (__ballot_sync(0xFFFFFFFFu, par.handle == kNone) >> (lane & 24u)) & 0xFFu; // a list ends at its first kNone
+            const uint32_t rx = par.x - first[0], ry = par.y - first[1], rz = par.z - first[2];
+            const bool used = !(ends & ((2u << q) - 1u)) && rx <= 1u && ry <= 1u && rz <= 1u;
+            uint4 sw[3] = {};
+            if (used) {
+                const uint4* p = reinterpret_cast<const uint4*>(item_ptr(d, par.handle));
+                sw[0] = p[0];
+                sw[1] = p[1];
+                sw[2] = p[2];
             }
-#pragma unroll
-            for (uint32_t r = 0; r < 3; ++r)
-                if (to[r] < 8u)
-                    leaves[to[r]][(lane + 32u * r) % kItemStride] = v[r];
+            uint4* leaves = reinterpret_cast<uint4*>(sh); // 8 slots of 12 words
             __syncwarp();
-        }
-        const uint32_t dx = ((lane >> 3) & 2u) | ((lane >> 2) & 1u), dy = ((lane >> 2) & 2u) | ((lane >> 1) & 1u), dz0 = lane & 1u;
-        const uint32_t vx = (w.x << 2) | dx, vy = (w.y << 2) | dy, vz0 = (w.z << 2) | dz0;
-        AxisTerm tx = {}, ty = {}, tz[2] = {};
-        if constexpr (TOOL != kToolTerrain) {
-            tx = axis_term<TOOL>(e, 0, vx);
-            ty = axis_term<TOOL>(e, 1, vy);
-            tz[0] = axis_term<TOOL>(e, 2, vz0);
-            tz[1] = axis_term<TOOL>(e, 2, vz0 + 2u);
-        }
-        uint32_t ops[2];
-        bool hasOld[2];
-        uint32_t oldMat[2] = { 0, 0 };
-        {
-            const uint32_t at = ((lane >> 3) & 1u) * 16u + (lane & 7u), half = lane < 16 ? lo : hi; // bit of voxel z1 = 0 in its mask word
-            bool keeps = false;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                hasOld[h] = (half >> (at + 8u * h)) & 1u;
-                ops[h] = TOOL == kToolTerrain ? OP_FILL : voxel_op<TOOL>(e, tx, ty, tz[h], hasOld[h]);
-                if (ops[h] != OP_KEEP)
-                    ++edited;
-                keeps |= hasOld[h] && (ops[h] == OP_KEEP || TOOL == SVDAG_TOOL_COPY || TOOL == SVDAG_TOOL_SPHERE_ERODE);
+            leaves[q * 3u] = make_uint4(0, 0, 0, 0);
+            __syncwarp();
+            if (used) {
+                uint4* to = leaves + ((rx * 2u + ry) * 2u + rz) * 3u;
+                to[0] = sw[0];
+                to[1] = sw[1];
+                to[2] = sw[2];
             }
-            if (TOOL != kToolTerrain && __any_sync(0xFFFFFFFFu, keeps)) { // materials that stay
-                const uint32_t before = lane < 16 ? 0u : (uint32_t)__popc(lo);
+            __syncwarp();
+            uint32_t slot[3][2], bits[3][2]; // per axis and voxel of the block: its part of the slot and of the mask bit
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const uint32_t rank = before + (uint32_t)__popc(half & ((1u << (at + 8u * h)) - 1u));
-                    oldMat[h] = (__shfl_sync(0xFFFFFFFFu, owRaw, 2u + (rank >> 3)) >> ((rank & 7u) * 4u)) & 0xFu;
+            for (uint32_t k = 0; k < 2; ++k) {
+                const uint32_t v[3] = { vx + k, vy + k, vz + k };
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    const int f = (int)v[a] + e.iDestToSource[a];
+                    const uint32_t u = (uint32_t)(f > 0 ? f : 0);
+                    slot[a][k] = ((u >> 2) - first[a]) << (2 - a);
+                    bits[a][k] = (((u & 1u) ? 4u : 0u) | ((u & 2u) ? 32u : 0u)) >> a;
                 }
             }
-        }
-        uint32_t px[4] = {}, lat[2] = {}; // noise paint: lerps along x, then along y
-        if constexpr (TOOL == SVDAG_TOOL_BOX_PAINT_NOISE) {
-            if (e.noiseCellLog2 >= 2) {
-                const uint32_t sx = smooth16u(cell_fraction(vx, e.noiseCellLog2)), sy = smooth16u(cell_fraction(vy, e.noiseCellLog2));
 #pragma unroll
-                for (uint32_t k = 0; k < 4; ++k)
-                    px[k] = lerp16u(corners[k], corners[k + 4], sx, 2u * sx);
-                lat[0] = lerp16u(px[0], px[2], sy, 2u * sy);
-                lat[1] = lerp16u(px[1], px[3], sy, 2u * sy);
-            }
-        }
-        uint32_t newMat[2];
-        bool set[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t dz = dz0 + 2u * h, vz = vz0 + 2u * h;
-            bool out = false;
-            uint32_t mat = 0;
-            if constexpr (TOOL == kToolTerrain) {
-                const uint32_t colH = __shfl_sync(0xFFFFFFFFu, th, dx * 4 + dz);
-                mat = scene_voxel(e.scene, vx, vy, vz, colH);
-                out = mat != SVDAG_NO_MATERIAL;
-            } else {
-                const uint32_t op = ops[h];
-                if (op == OP_FILL || op == OP_SUBDIVIDE) {
-                    if constexpr (TOOL == SVDAG_TOOL_BOX_ADD || TOOL == SVDAG_TOOL_SPHERE_ADD || TOOL == SVDAG_TOOL_SPHERE_PAINT) {
-                        out = true;
-                        mat = e.material;
-                    } else if constexpr (TOOL == SVDAG_TOOL_BOX_PAINT_NOISE) {
-                        out = true;
-                        if (e.noiseCellLog2 >= 2) { // a 4^3 leaf lies in one lattice cell
-                            const uint32_t sz = smooth16u(cell_fraction(vz, e.noiseCellLog2));
-                            mat = (lerp16u(lat[0], lat[1], sz, 2u * sz) >> 12) & 0xFu;
-                        } else {
-                            mat = noise_material(e.noiseSeed, e.noiseCellLog2, vx, vy, vz);
-                        }
-                    } else if constexpr (TOOL == SVDAG_TOOL_SPHERE_ERODE) { // get_new_value, :564-588
-                        const uint2* nb = erodeBuf[threadIdx.x >> 5];
-                        uint32_t count = 0;
-                        for (int oz = -1; oz <= 1; ++oz)
-                            for (int oy = -1; oy <= 1; ++oy)
-                                for (int ox = -1; ox <= 1; ++ox) {
-                                    if (ox == 0 && oy == 0 && oz == 0)
-                                        continue;
-                                    const int qx = (int)dx + ox, qy = (int)dy + oy, qz = (int)dz + oz; // -1 .. 4
-                                    const uint32_t li = (uint32_t)(((qx >> 2) + 1) * 9 + ((qy >> 2) + 1) * 3 + ((qz >> 2) + 1));
-                                    const uint32_t ix = (uint32_t)qx & 3u, iy = (uint32_t)qy & 3u, iz = (uint32_t)qz & 3u;
-                                    const uint32_t bit = ((ix & 1u) ? 4u : 0u) | ((iy & 1u) ? 2u : 0u) | ((iz & 1u) ? 1u : 0u) | ((ix & 2u) ? 32u : 0u)
-                                        | ((iy & 2u) ? 16u : 0u) | ((iz & 2u) ? 8u : 0u);
-                                    const uint2 m = nb[li];
-                                    count += ((bit < 32 ? m.x >> bit : m.y >> (bit - 32)) & 1u);
-                                }
-                        out = hasOld[h] && count > e.noiseSeed;
-                        mat = oldMat[h];
-                    } else if constexpr (TOOL == SVDAG_TOOL_COPY) { // get_new_value(uint3, optional, State), :225-252
-                        out = hasOld[h];
-                        mat = oldMat[h];
-                        int sx = (int)vx + e.iDestToSource[0], sy = (int)vy + e.iDestToSource[1], sz = (int)vz + e.iDestToSource[2];
-                        sx = sx > 0 ? sx : 0;
-                        sy = sy > 0 ? sy : 0;
-                        sz = sz > 0 ? sz : 0;
-                        const uint32_t ux = (uint32_t)sx, uy = (uint32_t)sy, uz = (uint32_t)sz;
-                        const uint32_t* src = copyBuf[threadIdx.x >> 5][(((ux >> 2) - base[0]) * 2u + ((uy >> 2) - base[1])) * 2u + ((uz >> 2) - base[2])];
-                        const uint32_t bitIdx = ((ux & 1u) ? 4u : 0u) | ((uy & 1u) ? 2u : 0u) | ((uz & 1u) ? 1u : 0u) | ((ux & 2u) ? 32u : 0u)
-                            | ((uy & 2u) ? 16u : 0u) | ((uz & 2u) ? 8u : 0u);
-                        uint32_t m;
-                        if (leaf_get_material(src[0], src[1], src, bitIdx, m)) {
-                            out = true;
-                            mat = m;
-                        }
-                    } else { // removal tools
-                        out = false;
-                    }
-                } else if (op == OP_KEEP) {
-                    out = hasOld[h];
-                    mat = oldMat[h];
+            for (uint32_t j = 0; j < 8; ++j) {
+                const uint32_t sl = slot[0][j >> 2] + slot[1][(j >> 1) & 1u] + slot[2][j & 1u];
+                const uint32_t bit = bits[0][j >> 2] | bits[1][(j >> 1) & 1u] | bits[2][j & 1u];
+                const uint32_t* src = sh + sl * 12u;
+                uint32_t m;
+                if (((meets >> j) & 1u) && leaf_get_material(src[0], src[1], src, bit, m)) {
+                    given |= 1u << j;
+                    mats |= m << (4u * j);
                 }
             }
-            set[h] = out;
-            newMat[h] = mat;
+            nbyte = obyte | given;
         }
-        const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, set[0]), b1 = __ballot_sync(0xFFFFFFFFu, set[1]);
-        const uint32_t nlo = leaf_mask_lo(b0, b1), nhi = leaf_mask_hi(b0, b1);
-        uint32_t mine = lane == 0 ? nlo : nhi; // lanes 0..9: the words of the new leaf
-        if ((b0 & b1) == 0xFFFFFFFFu) {
-            // full: word 2 + k holds the materials of voxels 8k .. 8k+7, which eight lanes own
-            uint32_t m0 = newMat[0] << (4u * (lane & 7u)), m1 = newMat[1] << (4u * (lane & 7u));
+
+        // The lane's materials in voxel order, consecutive.
+        uint32_t stream = __funnelshift_r(old.a, old.b, old.shift), packed = 0, shift = 0;
 #pragma unroll
-            for (int o = 1; o < 8; o <<= 1) {
-                m0 |= __shfl_xor_sync(0xFFFFFFFFu, m0, o);
-                m1 |= __shfl_xor_sync(0xFFFFFFFFu, m1, o);
+        for (uint32_t j = 0; j < 8; ++j) {
+            const uint32_t m = (given >> j) & 1u ? (mats >> (4u * j)) & 0xFu : stream & 0xFu;
+            stream >>= (obyte >> j) & 1u ? 4 : 0;
+            if ((nbyte >> j) & 1u) {
+                packed |= m << shift;
+                shift += 4u;
             }
-            const uint32_t k = (lane - 2u) & 7u, from = (k >> 1) * 8u;
-            const uint32_t w0 = __shfl_sync(0xFFFFFFFFu, m0, from), w1 = __shfl_sync(0xFFFFFFFFu, m1, from);
-            if (lane >= 2)
-                mine = (k & 1u) ? w1 : w0;
-            // is_leaf_fully_filled (my_gpu_hash_dag.h:143-166): all 64 voxels set, one material
-            const uint32_t first = __shfl_sync(0xFFFFFFFFu, newMat[0], 0);
-            if (__all_sync(0xFFFFFFFFu, newMat[0] == first && newMat[1] == first) && lane == 0)
+        }
+        uint32_t part = nbyte << byteAt;
+        part |= __shfl_xor_sync(0xFFFFFFFFu, part, 1);
+        part |= __shfl_xor_sync(0xFFFFFFFFu, part, 2);
+        const uint32_t other = __shfl_xor_sync(0xFFFFFFFFu, part, 4);
+        const uint2 nm = q < 4u ? make_uint2(part, other) : make_uint2(other, part);
+        const bool fullMask = (nm.x & nm.y) == 0xFFFFFFFFu;
+        uint32_t word = packed; // material word q
+        if (__any_sync(0xFFFFFFFFu, !fullMask && (nm.x | nm.y) != 0u)) {
+            // lane s's nibbles start at its rank, in the word of that number and run into the next
+            const uint32_t rank = below(nm);
+            word = 0;
+#pragma unroll
+            for (uint32_t s = 0; s < 8; ++s) {
+                const uint32_t ps = __shfl_sync(0xFFFFFFFFu, packed, s, 8), rs = __shfl_sync(0xFFFFFFFFu, rank, s, 8);
+                const uint32_t sft = 4u * (rs & 7u), at = rs >> 3;
+                word |= at == q ? ps << sft : 0u;
+                word |= at + 1u == q ? __funnelshift_l(ps, 0u, sft) : 0u;
+            }
+        }
+        // is_leaf_fully_filled (my_gpu_hash_dag.h:143-166): all 64 voxels set, one material
+        if (__any_sync(0xFFFFFFFFu, fullMask)) {
+            const uint32_t m = __shfl_sync(0xFFFFFFFFu, word, 0, 8) & 0xFu;
+            const uint32_t same = __ballot_sync(0xFFFFFFFFu, fullMask && word == m * 0x11111111u);
+            if (q == 0 && ((same >> (lane & 24u)) & 0xFFu) == 0xFFu)
                 ++fullLeaves;
-        } else if ((b0 | b1) == 0u) {
-            mine = 0u;
-        } else {
-            // Pack the materials in voxel order through the warp's 64-byte slice of shared memory: clear,
-            // scatter one byte per set voxel at its rank, then lanes 2..9 each fold 8 bytes into a word of
-            // nibbles (LeafBuilder, my_gpu_base_dag.h:102-150).
-            const uint32_t below = (1u << lane) - 1u, group = 0xFFu << (lane & 24u), under = (1u << (lane & 24u)) - 1u;
-            const uint32_t off0 = __popc(b0 & below) + __popc(b1 & under), off1 = __popc(b0 & (under | group)) + __popc(b1 & below);
-            uint32_t* pw = packBuf[threadIdx.x >> 5];
-            uint8_t* pb = reinterpret_cast<uint8_t*>(pw);
-            if (lane < 16)
-                pw[lane] = 0u;
-            __syncwarp();
-            if (set[0])
-                pb[off0] = (uint8_t)newMat[0];
-            if (set[1])
-                pb[off1] = (uint8_t)newMat[1];
-            __syncwarp();
-            if (lane >= 2 && lane < kItemStride) {
-                unsigned long long x = reinterpret_cast<const unsigned long long*>(pw)[lane - 2];
-                x = (x | (x >> 4)) & 0x00FF00FF00FF00FFull;
-                x = (x | (x >> 8)) & 0x0000FFFF0000FFFFull;
-                x = (x | (x >> 16)) & 0x00000000FFFFFFFFull;
-                mine = (uint32_t)x;
-            }
-            __syncwarp(); // the buffer is reused by the next leaf
         }
-        uint32_t* outLeaf = reinterpret_cast<uint32_t*>(scratch + offN) + (size_t)i * kItemStride;
-        if (lane < kItemStride)
-            outLeaf[lane] = mine;
-        w = wn;
-        wn = wnn;
-        owRaw = owNext;
+        if (active) {
+            uint32_t* outLeaf = reinterpret_cast<uint32_t*>(scratch + offN) + (size_t)i * kItemStride;
+            if (q == 0)
+                *reinterpret_cast<uint2*>(outLeaf) = nm;
+            outLeaf[2u + q] = word;
+        }
+        w = w1;
+        w1 = w2;
+        w2 = w3;
+        om = om1;
+        om1 = om2;
+        old = old1;
     }
-    for (int o = 16; o > 0; o >>= 1)
+    for (int o = 16; o > 0; o >>= 1) {
         edited += __shfl_xor_sync(0xFFFFFFFFu, edited, o);
+        oldRead += __shfl_xor_sync(0xFFFFFFFFu, oldRead, o);
+        fullLeaves += __shfl_xor_sync(0xFFFFFFFFu, fullLeaves, o);
+    }
     if (lane == 0) {
         if (edited)
             atomicAdd(&E.edited, (unsigned long long)edited);
@@ -1298,6 +1365,8 @@ union NarrowShared {
         DevTable tables[kMaxLevels];
         uint32_t full[kMaxLevels], reps[kMaxLevels], ran[kMaxLevels], added;
     } merge;
+    uint4 align;
+    uint32_t leaves[kBlockThreads / 8 * leaf_shared_words<SVDAG_TOOL_COPY>()]; // the leaf phase of a block's edit
 };
 
 // GPU-clock stamps at the phase barriers (svdag_last_edit_phase_times).
@@ -1657,8 +1726,9 @@ __global__ void __launch_bounds__(256) k_build_level(DevDag d, const __grid_cons
 template <uint32_t TOOL>
 __global__ void __launch_bounds__(256) k_build_leaves(DevDag d, const __grid_constant__ DevEditor e, char* scratch, unsigned long long scratchBytes)
 {
+    __shared__ __align__(16) uint32_t shared[256 / 8 * leaf_shared_words<TOOL>()];
     chain_wait();
-    ph_build_leaves<TOOL>(d, e, scratch, scratchBytes);
+    ph_build_leaves<TOOL>(d, e, scratch, scratchBytes, shared);
 }
 __global__ void __launch_bounds__(256) k_fix_level(DevDag d, uint32_t level, uint32_t builder, char* scratch)
 {
@@ -1709,7 +1779,7 @@ __device__ __forceinline__ uint32_t block_build(const DevDag& d, const DevEditor
         __syncthreads();
         stamp(d, stampAt);
     }
-    ph_build_leaves<TOOL>(d, ed, scratch, scratchBytes);
+    ph_build_leaves<TOOL>(d, ed, scratch, scratchBytes, sh.leaves);
     __syncthreads();
     stamp(d, stampAt);
     return wide;
