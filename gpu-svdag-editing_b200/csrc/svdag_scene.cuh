@@ -61,16 +61,42 @@ __host__ __device__ inline uint32_t terrain_height_from_fbm(const SceneParams& p
     const long long norm = ((1ll << p.terrain.octaves) - 1) * 65536;
     return (uint32_t)(base + (range * f) / norm);
 }
+// lerp16 and smooth16 in 32-bit arithmetic for lattice values a, b in [0, 65535] and t in [0, 65535]:
+// floor((b - a) t / 2^16) = floor((b - a + 2^16) t / 2^16) - t, whose product is not negative and whose
+// high half one unsigned multiply gives; t * t fits 32 bits. `t2` is 2t.
+__host__ __device__ inline uint32_t mulhi32(uint32_t a, uint32_t b) { return (uint32_t)(((unsigned long long)a * b) >> 32); }
+__host__ __device__ inline uint32_t lerp16u(uint32_t a, uint32_t b, uint32_t t, uint32_t t2)
+{
+    return a - t + mulhi32(((b - a) << 15) + 0x80000000u, t2);
+}
+__host__ __device__ inline uint32_t smooth16u(uint32_t t) { return mulhi32(t * t, 3u * 65536u - 2u * t); }
+__host__ __device__ inline uint32_t cell_fraction(uint32_t v, uint32_t cellLog2) // of a coordinate in its cell, in 1/65536
+{
+    const uint32_t f = v & ((1u << cellLog2) - 1u);
+    return cellLog2 <= 16 ? f << (16 - cellLog2) : f >> (cellLog2 - 16);
+}
+// Corner values (x, z) = (0, 0), (1, 0), (0, 1), (1, 1) of the lattice cell (ix, iz) of octave o (terrain_lattice,
+// whose first rounds the corners share).
+__host__ __device__ inline void terrain_corners(const SceneParams& p, uint32_t ix, uint32_t iz, uint32_t o, uint32_t (&v)[4])
+{
+    const uint32_t h = scene_fmix32(p.terrain.seed * 0x9E3779B9u ^ (o * 0x85EBCA6Bu) ^ 0x68E31DA4u);
+    const uint32_t h0 = scene_fmix32(h ^ (ix * 0xC2B2AE35u)), h1 = scene_fmix32(h ^ ((ix + 1u) * 0xC2B2AE35u));
+    const uint32_t z0 = iz * 0x27D4EB2Fu, z1 = (iz + 1u) * 0x27D4EB2Fu;
+    v[0] = scene_fmix32(h0 ^ z0) >> 16;
+    v[1] = scene_fmix32(h1 ^ z0) >> 16;
+    v[2] = scene_fmix32(h0 ^ z1) >> 16;
+    v[3] = scene_fmix32(h1 ^ z1) >> 16;
+}
+__host__ __device__ inline uint32_t corners_at(const uint32_t (&v)[4], uint32_t sx, uint32_t sz)
+{
+    return lerp16u(lerp16u(v[0], v[1], sx, 2u * sx), lerp16u(v[2], v[3], sx, 2u * sx), sz, 2u * sz);
+}
 __host__ __device__ inline long long terrain_octave(const SceneParams& p, uint32_t x, uint32_t z, uint32_t o)
 {
     const uint32_t c = terrain_cell_log2(p, o);
-    const uint32_t ix = x >> c, iz = z >> c, m = (1u << c) - 1u;
-    const long long fx = c <= 16 ? (long long)((x & m) << (16 - c)) : (long long)((x & m) >> (c - 16));
-    const long long fz = c <= 16 ? (long long)((z & m) << (16 - c)) : (long long)((z & m) >> (c - 16));
-    const long long sx = smooth16(fx), sz = smooth16(fz);
-    const long long a = lerp16(terrain_lattice(p, ix, iz, o), terrain_lattice(p, ix + 1, iz, o), sx);
-    const long long b = lerp16(terrain_lattice(p, ix, iz + 1, o), terrain_lattice(p, ix + 1, iz + 1, o), sx);
-    return lerp16(a, b, sz);
+    uint32_t v[4];
+    terrain_corners(p, x >> c, z >> c, o, v);
+    return corners_at(v, smooth16u(cell_fraction(x, c)), smooth16u(cell_fraction(z, c)));
 }
 __host__ __device__ inline uint32_t terrain_height(const SceneParams& p, uint32_t x, uint32_t z)
 {
@@ -79,11 +105,12 @@ __host__ __device__ inline uint32_t terrain_height(const SceneParams& p, uint32_
         f += terrain_octave(p, x, z, o) << (p.terrain.octaves - 1 - o);
     return terrain_height_from_fbm(p, f);
 }
-// Conservative height bounds over the aligned footprint [x0, x0+s) x [z0, z0+s).
-__host__ __device__ inline void terrain_bounds(const SceneParams& p, uint32_t x0, uint32_t z0, uint32_t s, uint32_t& hlo, uint32_t& hhi)
+// Conservative bounds of the octaves o0, o0 + step, .. of the fBm sum over the aligned footprint
+// [x0, x0+s) x [z0, z0+s), added to lo and hi.
+__host__ __device__ inline void terrain_bounds_octaves(const SceneParams& p, uint32_t x0, uint32_t z0, uint32_t s, uint32_t o0, uint32_t step,
+    long long& lo, long long& hi)
 {
-    long long lo = 0, hi = 0;
-    for (uint32_t o = 0; o < p.terrain.octaves; ++o) {
+    for (uint32_t o = o0; o < p.terrain.octaves; o += step) {
         const uint32_t c = terrain_cell_log2(p, o);
         const uint32_t ix0 = x0 >> c, iz0 = z0 >> c;
         const uint32_t ix1 = ((x0 + s - 1) >> c) + 1, iz1 = ((z0 + s - 1) >> c) + 1;
@@ -92,17 +119,16 @@ __host__ __device__ inline void terrain_bounds(const SceneParams& p, uint32_t x0
             // Inside one lattice cell the field is bilinear in the (monotone) smoothstep weights, so
             // the extremes sit at the footprint corners; integer truncation of the three lerps moves a
             // value at most 2 units below the real bilinear value.
-            const uint32_t x1 = x0 + s - 1, z1 = z0 + s - 1;
-            const long long v0 = terrain_octave(p, x0, z0, o), v1 = terrain_octave(p, x1, z0, o);
-            const long long v2 = terrain_octave(p, x0, z1, o), v3 = terrain_octave(p, x1, z1, o);
-            vlo = v0 < v1 ? v0 : v1;
-            vlo = vlo < v2 ? vlo : v2;
-            vlo = vlo < v3 ? vlo : v3;
-            vhi = v0 > v1 ? v0 : v1;
-            vhi = vhi > v2 ? vhi : v2;
-            vhi = vhi > v3 ? vhi : v3;
-            vlo = vlo - 2 < 0 ? 0 : vlo - 2;
-            vhi = vhi + 2 > 65535 ? 65535 : vhi + 2;
+            uint32_t v[4];
+            terrain_corners(p, ix0, iz0, o, v);
+            const uint32_t sx0 = smooth16u(cell_fraction(x0, c)), sx1 = smooth16u(cell_fraction(x0 + s - 1, c));
+            const uint32_t sz0 = smooth16u(cell_fraction(z0, c)), sz1 = smooth16u(cell_fraction(z0 + s - 1, c));
+            const uint32_t v0 = corners_at(v, sx0, sz0), v1 = corners_at(v, sx1, sz0), v2 = corners_at(v, sx0, sz1), v3 = corners_at(v, sx1, sz1);
+            const uint32_t a0 = v0 < v1 ? v0 : v1, a1 = v2 < v3 ? v2 : v3, b0 = v0 > v1 ? v0 : v1, b1 = v2 > v3 ? v2 : v3;
+            vlo = (long long)(a0 < a1 ? a0 : a1) - 2;
+            vhi = (long long)(b0 > b1 ? b0 : b1) + 2;
+            vlo = vlo < 0 ? 0 : vlo;
+            vhi = vhi > 65535 ? 65535 : vhi;
         } else if ((unsigned long long)(ix1 - ix0 + 1) * (iz1 - iz0 + 1) > 64) {
             vlo = 0;
             vhi = 65535;
@@ -117,6 +143,12 @@ __host__ __device__ inline void terrain_bounds(const SceneParams& p, uint32_t x0
         lo += vlo << (p.terrain.octaves - 1 - o);
         hi += vhi << (p.terrain.octaves - 1 - o);
     }
+}
+// Conservative height bounds over that footprint.
+__host__ __device__ inline void terrain_bounds(const SceneParams& p, uint32_t x0, uint32_t z0, uint32_t s, uint32_t& hlo, uint32_t& hhi)
+{
+    long long lo = 0, hi = 0;
+    terrain_bounds_octaves(p, x0, z0, s, 0, 1, lo, hi);
     hlo = terrain_height_from_fbm(p, lo);
     hhi = terrain_height_from_fbm(p, hi);
 }
@@ -182,14 +214,13 @@ __host__ __device__ inline uint32_t scene_voxel(const SceneParams& p, uint32_t x
     return y < h ? terrain_material(p, y) : SVDAG_NO_MATERIAL;
 }
 
-// Classification of the node [p << depth, +2^depth)^3: 0 = Subdivide, 1 = Fill (*material), 2 = Empty.
-__host__ __device__ inline uint32_t scene_classify(const SceneParams& p, uint32_t px, uint32_t py, uint32_t pz, uint32_t depth,
-    uint32_t& material)
+// Classification of the node [p << depth, +2^depth)^3 whose footprint's heights lie in [hlo, hhi]:
+// 0 = Subdivide, 1 = Fill (*material), 2 = Empty.
+__host__ __device__ inline uint32_t scene_classify_bounded(const SceneParams& p, uint32_t px, uint32_t py, uint32_t pz, uint32_t depth,
+    uint32_t hlo, uint32_t hhi, uint32_t& material)
 {
     const uint32_t s = 1u << depth;
     const uint32_t x0 = px << depth, y0 = py << depth, z0 = pz << depth;
-    uint32_t hlo, hhi;
-    terrain_bounds(p, x0, z0, s, hlo, hhi);
     uint32_t terrainOp = 0, terrainMat = 0;
     if (y0 >= hhi) {
         terrainOp = 2;
@@ -231,6 +262,13 @@ __host__ __device__ inline uint32_t scene_classify(const SceneParams& p, uint32_
     }
     material = terrainMat;
     return terrainOp;
+}
+__host__ __device__ inline uint32_t scene_classify(const SceneParams& p, uint32_t px, uint32_t py, uint32_t pz, uint32_t depth,
+    uint32_t& material)
+{
+    uint32_t hlo, hhi;
+    terrain_bounds(p, px << depth, pz << depth, 1u << depth, hlo, hhi);
+    return scene_classify_bounded(p, px, py, pz, depth, hlo, hhi, material);
 }
 
 } // namespace svdag
