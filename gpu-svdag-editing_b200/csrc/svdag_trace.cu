@@ -23,14 +23,19 @@ struct RayF {
 __device__ __forceinline__ float cmaxf(float a, float b) { return a > b ? a : b; }
 __device__ __forceinline__ float cminf(float a, float b) { return a < b ? a : b; }
 
+// float(v) for v < 2^23 and 2^e for small e, by the exponent field: exact, and on the pipes that add
+// instead of the conversion unit, which takes 16 lanes a clock.
+__device__ __forceinline__ float coord_float(uint32_t v) { return __uint_as_float(0x4B000000u + v) - 8388608.0f; }
+__device__ __forceinline__ float pow2_float(uint32_t e) { return __uint_as_float((127u + e) << 23); }
+
 // compute_intersection_mask, tracer.cu:56-173 (device max/min of two floats are fmaxf/fminf; the
 // vector max/min of cuda_math.h are the ternary forms).
 __device__ __forceinline__ uint32_t intersection_mask(bool isRoot, uint32_t level, uint32_t px, uint32_t py, uint32_t pz, uint32_t levels,
     const RayF& r, float rayTmax = 3.402823466e+38f)
 {
     const uint32_t shift = levels - level;
-    const float radius = float(1u << (shift - 1));
-    const float cx = radius + float(px << shift), cy = radius + float(py << shift), cz = radius + float(pz << shift);
+    const float radius = pow2_float(shift - 1u);
+    const float cx = radius + coord_float(px << shift), cy = radius + coord_float(py << shift), cz = radius + coord_float(pz << shift);
     const float rx = cx - r.ox, ry = cy - r.oy, rz = cz - r.oz;
     const float tmx = rx * r.ix, tmy = ry * r.iy, tmz = rz * r.iz;
     float tmin, tmax;
@@ -85,13 +90,10 @@ __device__ __forceinline__ uint32_t next_child(uint32_t order, uint32_t mask)
 
 __device__ __forceinline__ uint32_t first_child_mask(uint32_t lo, uint32_t hi) // Leaf::get_first_child_mask, base_dag.h:16-52
 {
-    uint32_t out = 0;
-#pragma unroll
-    for (uint32_t i = 0; i < 4; ++i) {
-        out |= ((lo >> (8 * i)) & 0xFFu) ? (1u << i) : 0u;
-        out |= ((hi >> (8 * i)) & 0xFFu) ? (1u << (i + 4)) : 0u;
-    }
-    return out;
+    // bit 7 of each byte set where the byte is not zero (the adds carry within a byte only), then bits 7, 15,
+    // 23, 31 -> 28..31: the partial products of the multiply never overlap
+    const auto bytes = [](uint32_t v) { return (((((v & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | v) & 0x80808080u) * 0x00204081u) >> 28; };
+    return bytes(lo) | (bytes(hi) << 4);
 }
 
 // Whether the ray meets the box [b0..b2] x [b3..b5] at some t >= 0 (slab test; a NaN from a zero
@@ -425,13 +427,14 @@ __device__ __forceinline__ uint32_t to_rgb888(float r, float g, float b) // Colo
 __global__ void __launch_bounds__(256) k_shade(DevDag d, svdag_trace_params tp, ShadeDev sp, svdag_hit* hits, uint32_t* rgba, float* sunOut,
     float* aoOut)
 {
-    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t y = blockIdx.y * blockDim.y + threadIdx.y;
+    // 8 x 4 pixel tiles per warp, as in k_trace
+    const uint32_t tix = threadIdx.y * 32u + threadIdx.x, tw = tix >> 5, tl = tix & 31u;
+    const uint32_t x = blockIdx.x * 32u + (tw & 3u) * 8u + (tl & 7u);
+    const uint32_t y = blockIdx.y * 8u + (tw >> 2) * 4u + (tl >> 3);
     __shared__ uint32_t sIndex[kMaxLevels][256];
     __shared__ uint32_t sMasks[kMaxLevels][256];
     if (x >= tp.width || y >= tp.height)
         return;
-    const uint32_t tix = threadIdx.y * blockDim.x + threadIdx.x;
     const size_t i = (size_t)y * tp.width + x;
     svdag_hit& si = hits[i];
     const bool hit = si.path[0] != 0 || si.path[1] != 0 || si.path[2] != 0;
