@@ -23,29 +23,41 @@ struct RayF {
 __device__ __forceinline__ float cmaxf(float a, float b) { return a > b ? a : b; }
 __device__ __forceinline__ float cminf(float a, float b) { return a < b ? a : b; }
 
-// float(v) for v < 2^23 and 2^e for small e, by the exponent field: exact, and on the pipes that add
-// instead of the conversion unit, which takes 16 lanes a clock.
-__device__ __forceinline__ float coord_float(uint32_t v) { return __uint_as_float(0x4B000000u + v) - 8388608.0f; }
+// 2^e for small e, by the exponent field.
 __device__ __forceinline__ float pow2_float(uint32_t e) { return __uint_as_float((127u + e) << 23); }
+// Traversals keep a node's corner coordinates (below 2^23) with the bits of the float 2^23 over them: the
+// float value is then one exact subtraction, and no conversion (16 lanes a clock) nor shift is needed.
+constexpr uint32_t kCoordBias = 0x4B000000u;
+__device__ __forceinline__ float coord_float(uint32_t biased) { return __uint_as_float(biased) - 8388608.0f; }
 
-// compute_intersection_mask, tracer.cu:56-173 (device max/min of two floats are fmaxf/fminf; the
-// vector max/min of cuda_math.h are the ternary forms).
-__device__ __forceinline__ uint32_t intersection_mask(bool isRoot, uint32_t level, uint32_t px, uint32_t py, uint32_t pz, uint32_t levels,
-    const RayF& r, float rayTmax = 3.402823466e+38f)
+// A ray all of whose inverse direction components are at most 1e30 in magnitude: every product and sum of its
+// intersection tests is finite, so no NaN reaches a comparison.
+__device__ __forceinline__ bool ray_tame(const RayF& r) { return fabsf(r.ix) <= 1e30f && fabsf(r.iy) <= 1e30f && fabsf(r.iz) <= 1e30f; }
+
+// compute_intersection_mask, tracer.cu:56-173, of the node of size 2^shift with the biased corner (X, Y, Z)
+// (device max/min of two floats are fmaxf/fminf; the vector max/min of cuda_math.h are the ternary forms,
+// which differ from them on NaN only: TAME rays take the one-instruction forms).
+template <bool TAME>
+__device__ __forceinline__ uint32_t intersection_mask(bool isRoot, uint32_t shift, uint32_t X, uint32_t Y, uint32_t Z, const RayF& r,
+    float rayTmax = 3.402823466e+38f)
 {
-    const uint32_t shift = levels - level;
     const float radius = pow2_float(shift - 1u);
-    const float cx = radius + coord_float(px << shift), cy = radius + coord_float(py << shift), cz = radius + coord_float(pz << shift);
+    const float cx = radius + coord_float(X), cy = radius + coord_float(Y), cz = radius + coord_float(Z);
     const float rx = cx - r.ox, ry = cy - r.oy, rz = cz - r.oz;
     const float tmx = rx * r.ix, tmy = ry * r.iy, tmz = rz * r.iz;
     float tmin, tmax;
     {
         const float sx = radius * fabsf(r.ix), sy = radius * fabsf(r.iy), sz = radius * fabsf(r.iz);
-        tmin = fmaxf(cmaxf(tmx - sx, cmaxf(tmy - sy, tmz - sz)), 0.0f);
-        tmax = cminf(tmx + sx, cminf(tmy + sy, tmz + sz));
+        if constexpr (TAME) {
+            tmin = fmaxf(fmaxf(tmx - sx, fmaxf(tmy - sy, tmz - sz)), 0.0f);
+            tmax = fminf(fminf(tmx + sx, fminf(tmy + sy, tmz + sz)), rayTmax);
+        } else {
+            tmin = fmaxf(cmaxf(tmx - sx, cmaxf(tmy - sy, tmz - sz)), 0.0f);
+            tmax = cminf(tmx + sx, cminf(tmy + sy, tmz + sz));
+            tmin = fmaxf(tmin, 0.0f); // ray.tmin
+            tmax = fminf(tmax, rayTmax); // ray.tmax
+        }
     }
-    tmin = fmaxf(tmin, 0.0f); // ray.tmin
-    tmax = fminf(tmax, rayTmax); // ray.tmax
     if (isRoot && (tmin >= tmax))
         return 0;
     uint32_t mask;
@@ -77,16 +89,37 @@ __device__ __forceinline__ uint32_t intersection_mask(bool isRoot, uint32_t leve
     return mask & 0xFFu;
 }
 
-// The first child ci = c ^ order (c = 0, 1, ...) whose bit is set (tracer.cu:45-54; mask != 0): the
-// mask is permuted so that bit c holds bit c ^ order, then the lowest set bit is taken.
-__device__ __forceinline__ uint32_t next_child(uint32_t order, uint32_t mask)
+// next[order][mask]: the first child ci = c ^ order (c = 0, 1, ...) whose bit is set (tracer.cu:45-54; mask != 0).
+// A lookup in shared memory in place of a dozen permutation instructions on the pipe that bounds the
+// traversal.
+struct alignas(8) NextChild {
+    uint8_t v[8 * 256];
+};
+constexpr NextChild make_next_child()
 {
-    uint32_t m = mask;
-    m = (order & 1u) ? (((m & 0x55u) << 1) | ((m >> 1) & 0x55u)) : m;
-    m = (order & 2u) ? (((m & 0x33u) << 2) | ((m >> 2) & 0x33u)) : m;
-    m = (order & 4u) ? (((m & 0x0Fu) << 4) | ((m >> 4) & 0x0Fu)) : m;
-    return ((uint32_t)__ffs(m) - 1u) ^ order;
+    NextChild t {};
+    for (uint32_t order = 0; order < 8; ++order)
+        for (uint32_t mask = 1; mask < 256; ++mask)
+            for (uint32_t c = 0; c < 8; ++c)
+                if ((mask >> (c ^ order)) & 1u) {
+                    t.v[order * 256 + mask] = (uint8_t)(c ^ order);
+                    break;
+                }
+    return t;
 }
+__device__ const NextChild kNextChild = make_next_child();
+
+// The node a traversal stands at. A bad handle (which only a bug could produce) latches SVDAG_ERR_CORRUPT
+// and reads as a node without children, so no child is ever looked up in it: a node with children needs
+// no second check.
+__device__ __forceinline__ const uint32_t* checked_item(const DevDag& d, uint32_t lastHandle, uint32_t h)
+{
+    if (h <= lastHandle)
+        return handle_ptr(d, h);
+    set_status(d.ctl, SVDAG_ERR_CORRUPT);
+    return kZeroItem;
+}
+__device__ __forceinline__ uint32_t last_handle(const DevDag& d) { return (uint32_t)((d.itemWords - 16ull) / kUnitWords); } // handle_ok
 
 __device__ __forceinline__ uint32_t first_child_mask(uint32_t lo, uint32_t hi) // Leaf::get_first_child_mask, base_dag.h:16-52
 {
@@ -108,6 +141,80 @@ __device__ __forceinline__ bool ray_meets_box(const RayF& r, const float* b)
     return tnear <= tfar;
 }
 
+// intersect_ray, tracer.cu:186-273: the first voxel on the ray and its material; leaves the coordinates as they
+// are when there is none. Stack in shared memory, [level][thread] so that a warp's accesses hit distinct
+// banks. Bound by the integer and compare pipe (75 % busy).
+template <bool TAME>
+__device__ __forceinline__ void first_hit(const DevDag& d, uint32_t root, const RayF& r, uint32_t (*sIndex)[256], uint32_t (*sMasks)[256],
+    const uint8_t* sNext, uint32_t tix, uint32_t& px, uint32_t& py, uint32_t& pz, uint32_t& material)
+{
+    const uint32_t levels = d.levels, LL = d.leafLevel, last = last_handle(d);
+    const uint8_t* next = sNext + 256u * ((r.dx < 0.f ? 4u : 0u) + (r.dy < 0.f ? 2u : 0u) + (r.dz < 0.f ? 1u : 0u));
+    uint32_t level = 0, X = kCoordBias, Y = kCoordBias, Z = kCoordBias, leafLo = 0, leafHi = 0;
+    uint32_t node = root;
+    uint32_t children = checked_item(d, last, root)[0] & 0xFFu;
+    uint32_t visit = children & intersection_mask<TAME>(true, levels, X, Y, Z, r);
+    // Bit l of `live`: the stack entry of level l still has children to visit. Ascending to the
+    // deepest such level below the current one is what the reference's pop loop does one level
+    // at a time (entries in between have nothing left); here it is one bit scan.
+    uint32_t live = 0;
+    for (;;) {
+        if (!visit) {
+            const uint32_t cand = live & ((1u << level) - 1u);
+            if (!cand)
+                return;
+            level = 31u - (uint32_t)__clz(cand);
+            node = sIndex[level][tix];
+            const uint32_t m = sMasks[level][tix];
+            children = m & 0xFFu;
+            visit = m >> 8;
+            const uint32_t corner = ~0u << (levels - level);
+            X &= corner;
+            Y &= corner;
+            Z &= corner;
+        }
+        const uint32_t child = next[visit];
+        visit &= ~(1u << child);
+        sIndex[level][tix] = node;
+        sMasks[level][tix] = children | (visit << 8);
+        live = visit ? (live | (1u << level)) : (live & ~(1u << level));
+        level++;
+        const uint32_t half = 1u << (levels - level);
+        X += (child >> 2) * half;
+        Y += ((child >> 1) & 1u) * half;
+        Z += (child & 1u) * half;
+        if (level == levels) {
+            px = X - kCoordBias;
+            py = Y - kCoordBias;
+            pz = Z - kCoordBias;
+            const uint32_t voxel = ((px & 1u) ? 4u : 0u) | ((py & 1u) ? 2u : 0u) | ((pz & 1u) ? 1u : 0u) | ((px & 2u) ? 32u : 0u)
+                | ((py & 2u) ? 16u : 0u) | ((pz & 2u) ? 8u : 0u); // mortonU32() & 63
+            const uint32_t* leaf = checked_item(d, last, node); // the leaf, since the levels inside it keep it
+            const unsigned long long m = (unsigned long long)leafLo | ((unsigned long long)leafHi << 32);
+            if ((m >> voxel) & 1ull) {
+                const uint32_t bit = __popcll(m & ((1ull << voxel) - 1ull)) * 4u;
+                material = (leaf[2 + (bit >> 5)] >> (bit & 31u)) & 0xFu;
+            }
+            return;
+        }
+        // The child's mask by level kind, then one intersection test for all lanes together (the
+        // branches only fetch; the mask arithmetic runs converged).
+        if (level <= LL) {
+            node = handle_ptr(d, node)[1 + __popc(children & ((1u << child) - 1u))];
+            const uint32_t* p = checked_item(d, last, node);
+            children = p[0] & 0xFFu;
+            if (level == LL) {
+                leafLo = p[0];
+                leafHi = p[1];
+                children = first_child_mask(leafLo, leafHi);
+            }
+        } else { // get_second_child_mask, base_dag.h:53-58
+            children = (((child & 4u) ? leafHi : leafLo) >> ((child & 3u) * 8u)) & 0xFFu;
+        }
+        visit = children & intersection_mask<TAME>(false, levels - level, X, Y, Z, r);
+    }
+}
+
 // Primary rays. With INCR the buffer holds the previous frame of the same camera and only pixels
 // whose ray meets one of `boxes` (the changed regions since that frame, grown by a margin) are traced
 // again. The traversal only ever inspects voxels within the intersection test's tolerance (1e-4) of
@@ -126,6 +233,12 @@ __global__ void __launch_bounds__(256) k_trace(DevDag d, svdag_trace_params p, s
     const uint32_t tw = (threadIdx.y * 32u + threadIdx.x) >> 5, tl = threadIdx.x & 31u;
     const uint32_t x = blockIdx.x * 32u + (tw & 3u) * 8u + (tl & 7u);
     const uint32_t y = blockIdx.y * 8u + (tw >> 2) * 4u + (tl >> 3);
+    __shared__ uint32_t sIndex[kMaxLevels][256];
+    __shared__ uint32_t sMasks[kMaxLevels][256]; // children | children left to visit << 8
+    __shared__ __align__(8) uint8_t sNext[8 * 256];
+    const uint32_t tix = threadIdx.y * blockDim.x + threadIdx.x;
+    reinterpret_cast<uint2*>(sNext)[tix] = reinterpret_cast<const uint2*>(kNextChild.v)[tix];
+    __syncthreads();
     if (x >= p.width || y >= p.height)
         return;
     // Ray setup in double (trace_paths, tracer.cu:403-405; normalize = (1 / length) * v).
@@ -146,87 +259,20 @@ __global__ void __launch_bounds__(256) k_trace(DevDag d, svdag_trace_params p, s
     r.iy = 1.0f / r.dy;
     r.iz = 1.0f / r.dz;
     if constexpr (INCR) {
-        bool touched = !(fabsf(r.ix) <= 1e30f && fabsf(r.iy) <= 1e30f && fabsf(r.iz) <= 1e30f);
+        bool touched = !ray_tame(r);
         for (uint32_t b = 0; b < nBoxes && !touched; ++b)
             touched = ray_meets_box(r, boxes + 6 * b);
         if (!touched)
             return;
     }
 
-    // intersect_ray, tracer.cu:186-273.
-    const uint32_t levels = d.levels, LL = d.leafLevel;
-    const uint32_t order = (r.dx < 0.f ? 4u : 0u) + (r.dy < 0.f ? 2u : 0u) + (r.dz < 0.f ? 1u : 0u);
-    // Traversal stack in shared memory, [level][thread] so that a warp's accesses hit distinct banks.
-    __shared__ uint32_t sIndex[kMaxLevels][256];
-    __shared__ uint32_t sMasks[kMaxLevels][256]; // childMask | visitMask << 8
-    const uint32_t tix = threadIdx.y * blockDim.x + threadIdx.x;
-    uint32_t level = 0, addr = 0, px = 0, py = 0, pz = 0, leafLo = 0, leafHi = 0;
-    uint32_t material = 0xFFFFFFFFu;
+    uint32_t px = 0, py = 0, pz = 0, material = 0xFFFFFFFFu;
     const uint32_t root = rootPtr ? *rootPtr : d.ctl->root;
     if (root != kNone) {
-        uint32_t cIndex = root;
-        uint32_t cChild = item_ptr(d, root)[0] & 0xFFu;
-        uint32_t cVisit = cChild & intersection_mask(true, 0, 0, 0, 0, levels, r);
-        // Bit l of `live`: the stack entry of level l still has children to visit. Ascending to the
-        // deepest such level below the current one is what the reference's pop loop does one level
-        // at a time (entries in between have nothing left); here it is one bit scan.
-        uint32_t live = 0;
-        for (;;) {
-            if (!cVisit) {
-                const uint32_t cand = live & ((1u << level) - 1u);
-                if (!cand) {
-                    px = py = pz = 0;
-                    break;
-                }
-                const uint32_t newLevel = 31u - (uint32_t)__clz(cand);
-                cIndex = sIndex[newLevel][tix];
-                const uint32_t m = sMasks[newLevel][tix];
-                cChild = m & 0xFFu;
-                cVisit = m >> 8;
-                const uint32_t up = level - newLevel;
-                px >>= up;
-                py >>= up;
-                pz >>= up;
-                level = newLevel;
-            }
-            const uint32_t nextChild = next_child(order, cVisit);
-            cVisit &= ~(1u << nextChild);
-            px = (px << 1) | ((nextChild >> 2) & 1u);
-            py = (py << 1) | ((nextChild >> 1) & 1u);
-            pz = (pz << 1) | (nextChild & 1u);
-            sIndex[level][tix] = cIndex;
-            sMasks[level][tix] = cChild | (cVisit << 8);
-            live = cVisit ? (live | (1u << level)) : (live & ~(1u << level));
-            level++;
-            if (level == levels) {
-                const uint32_t voxel = ((px & 1u) ? 4u : 0u) | ((py & 1u) ? 2u : 0u) | ((pz & 1u) ? 1u : 0u) | ((px & 2u) ? 32u : 0u)
-                    | ((py & 2u) ? 16u : 0u) | ((pz & 2u) ? 8u : 0u); // mortonU32() & 63
-                const uint32_t* leaf = item_ptr(d, addr);
-                const unsigned long long m = (unsigned long long)leafLo | ((unsigned long long)leafHi << 32);
-                if ((m >> voxel) & 1ull) {
-                    const uint32_t bit = __popcll(m & ((1ull << voxel) - 1ull)) * 4u;
-                    material = (leaf[2 + (bit >> 5)] >> (bit & 31u)) & 0xFu;
-                }
-                break;
-            }
-            // The child's mask by level kind, then one intersection test for all lanes together (the
-            // branches only fetch; the mask arithmetic runs converged).
-            if (level < LL) {
-                const uint32_t* node = item_ptr(d, cIndex);
-                cIndex = node[1 + __popc(cChild & ((1u << nextChild) - 1u))];
-                cChild = item_ptr(d, cIndex)[0] & 0xFFu;
-            } else if (level == LL) {
-                const uint32_t* node = item_ptr(d, cIndex);
-                addr = node[1 + __popc(cChild & ((1u << nextChild) - 1u))];
-                const uint32_t* lp = item_ptr(d, addr);
-                leafLo = lp[0];
-                leafHi = lp[1];
-                cChild = first_child_mask(leafLo, leafHi);
-            } else { // get_second_child_mask, base_dag.h:53-58
-                cChild = (((nextChild & 4u) ? leafHi : leafLo) >> ((nextChild & 3u) * 8u)) & 0xFFu;
-            }
-            cVisit = cChild & intersection_mask(false, level, px, py, pz, levels, r);
-        }
+        if (ray_tame(r))
+            first_hit<true>(d, root, r, sIndex, sMasks, sNext, tix, px, py, pz, material);
+        else
+            first_hit<false>(d, root, r, sIndex, sMasks, sNext, tix, px, py, pz, material);
     }
     if (px == 0 && py == 0 && pz == 0)
         material = 0xFFFFFFFFu; // a miss has no material (Path::is_null, path.h:61-64)
@@ -281,59 +327,64 @@ struct ShadeDev {
 
 // intersect_ray_node_out_of_order, tracer.cu:275-352: whether any voxel lies on the ray within
 // [0, tmax]; children are taken highest index first, whatever the ray's direction.
+template <bool TAME>
+__device__ __forceinline__ bool any_hit_as(const DevDag& d, uint32_t root, const RayF& r, float tmax, uint32_t (*sIndex)[256],
+    uint32_t (*sMasks)[256], uint32_t tix)
+{
+    const uint32_t levels = d.levels, LL = d.leafLevel, last = last_handle(d);
+    uint32_t level = 0, X = kCoordBias, Y = kCoordBias, Z = kCoordBias, leafLo = 0, leafHi = 0;
+    uint32_t node = root;
+    uint32_t children = checked_item(d, last, root)[0] & 0xFFu;
+    uint32_t visit = children & intersection_mask<TAME>(true, levels, X, Y, Z, r, tmax);
+    uint32_t live = 0; // as in first_hit: bit l set while stack level l has children left
+    for (;;) {
+        if (!visit) {
+            const uint32_t cand = live & ((1u << level) - 1u);
+            if (!cand)
+                return false;
+            level = 31u - (uint32_t)__clz(cand);
+            node = sIndex[level][tix];
+            const uint32_t m = sMasks[level][tix];
+            children = m & 0xFFu;
+            visit = m >> 8;
+            const uint32_t corner = ~0u << (levels - level);
+            X &= corner;
+            Y &= corner;
+            Z &= corner;
+        }
+        const uint32_t child = 31u - (uint32_t)__clz(visit);
+        visit &= ~(1u << child);
+        sIndex[level][tix] = node;
+        sMasks[level][tix] = children | (visit << 8);
+        live = visit ? (live | (1u << level)) : (live & ~(1u << level));
+        level++;
+        if (level == levels)
+            return true;
+        const uint32_t half = 1u << (levels - level);
+        X += (child >> 2) * half;
+        Y += ((child >> 1) & 1u) * half;
+        Z += (child & 1u) * half;
+        if (level <= LL) {
+            node = handle_ptr(d, node)[1 + __popc(children & ((1u << child) - 1u))];
+            const uint32_t* p = checked_item(d, last, node);
+            children = p[0] & 0xFFu;
+            if (level == LL) {
+                leafLo = p[0];
+                leafHi = p[1];
+                children = first_child_mask(leafLo, leafHi);
+            }
+        } else {
+            children = (((child & 4u) ? leafHi : leafLo) >> ((child & 3u) * 8u)) & 0xFFu;
+        }
+        visit = children & intersection_mask<TAME>(false, levels - level, X, Y, Z, r, tmax);
+    }
+}
 __device__ bool any_hit(const DevDag& d, uint32_t root, const RayF& r, float tmax, uint32_t (*sIndex)[256], uint32_t (*sMasks)[256],
     uint32_t tix)
 {
     if (root == kNone)
         return false;
-    const uint32_t levels = d.levels, LL = d.leafLevel;
-    uint32_t level = 0, px = 0, py = 0, pz = 0, leafLo = 0, leafHi = 0;
-    uint32_t cIndex = root;
-    uint32_t cChild = item_ptr(d, root)[0] & 0xFFu;
-    uint32_t cVisit = cChild & intersection_mask(true, 0, 0, 0, 0, levels, r, tmax);
-    uint32_t live = 0; // as in k_trace: bit l set while stack level l has children left
-    for (;;) {
-        if (!cVisit) {
-            const uint32_t cand = live & ((1u << level) - 1u);
-            if (!cand)
-                return false;
-            const uint32_t newLevel = 31u - (uint32_t)__clz(cand);
-            cIndex = sIndex[newLevel][tix];
-            const uint32_t m = sMasks[newLevel][tix];
-            cChild = m & 0xFFu;
-            cVisit = m >> 8;
-            const uint32_t up = level - newLevel;
-            px >>= up;
-            py >>= up;
-            pz >>= up;
-            level = newLevel;
-        }
-        const uint32_t nextChild = 31u - (uint32_t)__clz(cVisit);
-        cVisit &= ~(1u << nextChild);
-        px = (px << 1) | ((nextChild >> 2) & 1u);
-        py = (py << 1) | ((nextChild >> 1) & 1u);
-        pz = (pz << 1) | (nextChild & 1u);
-        sIndex[level][tix] = cIndex;
-        sMasks[level][tix] = cChild | (cVisit << 8);
-        live = cVisit ? (live | (1u << level)) : (live & ~(1u << level));
-        level++;
-        if (level == levels)
-            return true;
-        if (level < LL) {
-            const uint32_t* node = item_ptr(d, cIndex);
-            cIndex = node[1 + __popc(cChild & ((1u << nextChild) - 1u))];
-            cChild = item_ptr(d, cIndex)[0] & 0xFFu;
-        } else if (level == LL) {
-            const uint32_t* node = item_ptr(d, cIndex);
-            const uint32_t* lp = item_ptr(d, node[1 + __popc(cChild & ((1u << nextChild) - 1u))]);
-            leafLo = lp[0];
-            leafHi = lp[1];
-            cChild = first_child_mask(leafLo, leafHi);
-        } else {
-            cChild = (((nextChild & 4u) ? leafHi : leafLo) >> ((nextChild & 3u) * 8u)) & 0xFFu;
-        }
-        cVisit = cChild & intersection_mask(false, level, px, py, pz, levels, r, tmax);
-    }
+    return ray_tame(r) ? any_hit_as<true>(d, root, r, tmax, sIndex, sMasks, tix) : any_hit_as<false>(d, root, r, tmax, sIndex, sMasks, tix);
 }
 
 __device__ __forceinline__ RayF make_rayf(float ox, float oy, float oz, float dx, float dy, float dz) // Ray::create, tracer.cu:32-41
