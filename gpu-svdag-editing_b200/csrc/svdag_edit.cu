@@ -2580,10 +2580,10 @@ svdag_status build_scene_untiled(svdag_ctx* ctx, const DevEditor& ed, cudaStream
         uint32_t buckets[kNumClasses];
         for (uint32_t c = 0; c < kNumClasses; ++c) {
             const unsigned long long items = (unsigned long long)reps[c] + SVDAG_NUM_MATERIALS;
-            buckets[c] = (uint32_t)std::max<unsigned long long>(min_level_buckets(ctx), (items + ctx->loadFactor - 1) / ctx->loadFactor);
+            buckets[c] = (uint32_t)std::max<unsigned long long>(1, (items + ctx->loadFactor - 1) / ctx->loadFactor);
         }
         svdag_table& t = ctx->levelTables[level];
-        SVDAG_TRY(alloc_table(ctx, &t, level == (int)LL ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets, s, true));
+        SVDAG_TRY(alloc_level_table(ctx, &t, level == (int)LL ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets, s));
         t.level = level;
         SVDAG_TRY(upload_tables(ctx, s));
         SVDAG_TRY(insert_canonical(ctx, (uint32_t)level, s));

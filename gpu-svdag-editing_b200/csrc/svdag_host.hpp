@@ -88,7 +88,7 @@ svdag_status insert_canonical(svdag_ctx* ctx, uint32_t level, cudaStream_t s);
 svdag_status upload_tables(svdag_ctx* ctx, cudaStream_t s);
 svdag_status read_status(svdag_ctx* ctx, cudaStream_t s);
 void reset_level_tables(svdag_ctx* ctx);
-uint32_t min_level_buckets(const svdag_ctx* ctx); // fewest buckets of a class of a level table
+svdag_status alloc_level_table(svdag_ctx* ctx, svdag_table* t, uint32_t kind, const uint32_t* bucketsPerClass, cudaStream_t s);
 // Find-or-insert of keys that are pairwise distinct (no batch dedup) into a level table.
 svdag_status find_or_insert_distinct(svdag_ctx* ctx, uint32_t level, const uint32_t* keys, const uint32_t* offsets, uint32_t n,
     unsigned long long totalWords, uint32_t* out, cudaStream_t s);

@@ -137,9 +137,9 @@ svdag_status load_snapshot(svdag_ctx* ctx, const uint32_t* words, const uint64_t
         }
         uint32_t buckets[kNumClasses];
         for (uint32_t c = 0; c < kNumClasses; ++c)
-            buckets[c] = (uint32_t)std::max<unsigned long long>(min_level_buckets(ctx), (perClass[c] + SVDAG_NUM_MATERIALS + ctx->loadFactor - 1) / ctx->loadFactor);
+            buckets[c] = (uint32_t)std::max<unsigned long long>(1, (perClass[c] + SVDAG_NUM_MATERIALS + ctx->loadFactor - 1) / ctx->loadFactor);
         svdag_table& t = ctx->levelTables[level];
-        SVDAG_TRY(alloc_table(ctx, &t, leaf ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets, s, true));
+        SVDAG_TRY(alloc_level_table(ctx, &t, leaf ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets, s));
         t.level = (uint32_t)level;
         SVDAG_TRY(upload_tables(ctx, s));
         SVDAG_TRY(insert_canonical(ctx, (uint32_t)level, s));

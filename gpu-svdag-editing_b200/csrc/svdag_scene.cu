@@ -220,12 +220,13 @@ struct TiledBuild {
     unsigned long long topBytes;
 
     // Allocates the level tables (bottom-up, canonical items first) and makes them current.
-    svdag_status alloc_tables(const std::vector<std::vector<uint32_t>>& buckets, cudaStream_t s)
+    svdag_status alloc_tables(const std::vector<std::vector<uint32_t>>& buckets, bool provisional, cudaStream_t s)
     {
         const uint32_t LL = ctx->cfg.levels - 2;
         for (int level = (int)LL; level >= 0; --level) {
             svdag_table& t = ctx->levelTables[level];
-            SVDAG_TRY(alloc_table(ctx, &t, level == (int)LL ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets[level].data(), s, true));
+            const uint32_t kind = level == (int)LL ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE;
+            SVDAG_TRY(provisional ? alloc_table(ctx, &t, kind, buckets[level].data(), s, true) : alloc_level_table(ctx, &t, kind, buckets[level].data(), s));
             t.level = level;
             SVDAG_TRY(insert_canonical(ctx, (uint32_t)level, s));
         }
@@ -383,18 +384,18 @@ svdag_status run_scene_build(svdag_ctx* ctx, const svdag_terrain_params* p, cuda
     }
     uint32_t root = kNone;
     SVDAG_TRY(reset_dag(ctx, s));
-    SVDAG_TRY(tb.alloc_tables(buckets, s));
+    SVDAG_TRY(tb.alloc_tables(buckets, true, s));
     SVDAG_TRY(tb.build(root, s));
     unsigned long long* counters = reinterpret_cast<unsigned long long*>(tb.top + topBytes - 256);
     for (uint32_t level = 0; level <= LL; ++level) {
         unsigned long long per[kNumClasses];
         SVDAG_TRY(table_class_counts(ctx, ctx->levelTables[level], per, counters, s));
         for (uint32_t c = 0; c < kNumClasses; ++c)
-            buckets[level][c] = (uint32_t)std::max<unsigned long long>(min_level_buckets(ctx), (per[c] + ctx->loadFactor - 1) / ctx->loadFactor);
+            buckets[level][c] = (uint32_t)std::max<unsigned long long>(1, (per[c] + ctx->loadFactor - 1) / ctx->loadFactor);
     }
     // Final pass into exactly sized tables.
     SVDAG_TRY(reset_dag(ctx, s));
-    SVDAG_TRY(tb.alloc_tables(buckets, s));
+    SVDAG_TRY(tb.alloc_tables(buckets, false, s));
     SVDAG_TRY(tb.build(root, s));
     SVDAG_CUDA(cudaMemcpyAsync(&ctx->ctl->root, &root, sizeof(root), cudaMemcpyHostToDevice, s));
     SVDAG_CUDA(cudaStreamSynchronize(s));

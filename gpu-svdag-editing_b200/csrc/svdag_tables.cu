@@ -123,20 +123,24 @@ void reset_level_tables(svdag_ctx* ctx)
         t = svdag_table {};
 }
 
-// Fewest buckets of each size class of a level table. Every edit leaves a new version of each node on
+// Allocates a level table of at least the given bucket counts. Every edit leaves a new version of each node on
 // its path, so the table of an upper level grows with the edits whatever its scene held: sized from
 // the scene alone, the root's table has one bucket of the class all its versions fall in, a group of
 // edits takes turns on that bucket's lock and each one walks its chain. 256 scattered small edits at
-// depth 15 took 5.03 ms that way and take 2.79 ms with these tables. All minimum
-// tables together take at most 1/32 of the region, and 2048 buckets hold 32768 versions at the default
-// load.
-uint32_t min_level_buckets(const svdag_ctx* ctx)
+// depth 15 took 5.03 ms that way and 2.79 ms with these tables. 2048 buckets hold 32768 versions at the
+// default load; all levels' minimum together takes at most 1/32 of the region.
+svdag_status alloc_level_table(svdag_ctx* ctx, svdag_table* t, uint32_t kind, const uint32_t* bucketsPerClass, cudaStream_t s)
 {
     unsigned long long row = 0; // bytes of one bucket of every class
     for (uint32_t k = 2; k < 2 + kNumClasses; ++k)
         row += slab_bytes(k);
     const unsigned long long region = ctx->itemWords * 4ull + ctx->headerCount * 32ull;
-    return (uint32_t)std::min<unsigned long long>(2048, std::max<unsigned long long>(1, region / 32 / (ctx->cfg.levels - 1) / row));
+    const uint32_t least = (uint32_t)std::min<unsigned long long>(2048, region / 32 / (ctx->cfg.levels - 1) / row);
+    uint32_t buckets[kNumClasses];
+    for (uint32_t c = 0; c < kNumClasses; ++c)
+        buckets[c] = std::max(bucketsPerClass[c], least);
+    const svdag_status st = alloc_table(ctx, t, kind, buckets, s, true);
+    return st == SVDAG_ERR_OOM ? alloc_table(ctx, t, kind, bucketsPerClass, s, true) : st; // a region that is nearly full
 }
 
 // Default bucket counts for a level that was not sized by a scene build: the surface of a scene
@@ -152,8 +156,8 @@ svdag_status ensure_level_tables(svdag_ctx* ctx, cudaStream_t s)
         const unsigned long long expect = std::min<unsigned long long>(1ull << (2 * (level + 1)), 1ull << 20);
         uint32_t buckets[kNumClasses];
         for (uint32_t c = 0; c < kNumClasses; ++c)
-            buckets[c] = (uint32_t)std::max<unsigned long long>(min_level_buckets(ctx), expect / (4ull * ctx->loadFactor));
-        SVDAG_TRY(alloc_table(ctx, &t, level == (int)leaf ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets, s, true));
+            buckets[c] = (uint32_t)std::max<unsigned long long>(1, expect / (4ull * ctx->loadFactor));
+        SVDAG_TRY(alloc_level_table(ctx, &t, level == (int)leaf ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets, s));
         t.level = level;
         SVDAG_TRY(insert_canonical(ctx, (uint32_t)level, s));
         created = true;
