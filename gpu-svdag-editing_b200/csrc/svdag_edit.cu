@@ -2357,8 +2357,10 @@ constexpr unsigned long long kSubtreeScratch = 16ull << 20; // scratch slice of 
 // k_edit_subtrees, k_edit_spines), where that is the faster of the two. Measured for spheres and boxes
 // at depth 14: a chain takes 55 us and 5 us more per 1000 estimated leaves (radius 9: 68, radius 70: 113);
 // a group takes 60 us for its paths and its slowest block, which is 55 us and 35 us more per 1000
-// leaves (radius 20: 90, radius 70: 390-590). An edit alone in the one-block kernel is never faster than
-// its chain (radius 1: 57 against 55 us; radius 45: 200 against 98).
+// leaves (radius 20: 90, radius 70: 390-590). An edit alone runs in the one-block kernel, where the context
+// asks for it, only up to 400 leaves, where one launch takes what the chain takes (radius 9: 68 against
+// 68 us; radius 20: 92 against 80, radius 45: 200 against 98).
+constexpr double kBlockAloneLeaves = 400.0;
 double chain_us(double leaves) { return 55.0 + 0.005 * leaves; }
 double group_us(double mostLeaves) { return 60.0 + 55.0 + 0.035 * mostLeaves; }
 
@@ -2504,7 +2506,7 @@ svdag_status run_edit(svdag_ctx* ctx, const svdag_edit* e, cudaStream_t s)
     DevEditor eds[2];
     const int n = expand_edit(ctx, *e, eds);
     for (int i = 0; i < n; ++i) {
-        if (ctx->persistentLeaves > 0 && estimate_leaves(eds[i]) <= ctx->persistentLeaves)
+        if (estimate_leaves(eds[i]) <= std::min(ctx->persistentLeaves, kBlockAloneLeaves))
             SVDAG_TRY(launch_single_fused(ctx, eds[i], s));
         else
             SVDAG_TRY(launch_pipeline(ctx, eds[i], s, nullptr));

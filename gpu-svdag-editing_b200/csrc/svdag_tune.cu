@@ -135,15 +135,15 @@ svdag_status tune_edits(svdag_ctx* ctx, const svdag_edit* edits, uint32_t n, svd
     double sum[kBuckets][2] = {}, cnt[kBuckets][2] = {};
     std::vector<Timer> timers(2 * (size_t)n);
     std::vector<int> bucketOf(2 * (size_t)n, -1), formOf(2 * (size_t)n, 0);
-    // The first launch of a tool in a form may capture and instantiate its graph or load the kernel:
-    // it is applied like the others but left out of the statistics (bucket -1).
+    // The first launch of a tool in a form may load its kernels: it is applied like the others but left
+    // out of the statistics (bucket -1).
     bool seen[2][SVDAG_NUM_TOOLS] = {};
     size_t used = 0;
     for (uint32_t i = 0; i < n; ++i) {
         DevEditor eds[2];
         const int m = expand_edit(ctx, edits[i], eds);
         for (int j = 0; j < m; ++j) {
-            const int form = (int)((i + j) & 1u); // 0 graph, 1 persistent
+            const int form = (int)((i + j) & 1u); // 0 chain of launches, 1 one block
             const double est = estimate_leaves(eds[j]);
             int b = 0;
             while (b < kBuckets - 1 && est >= upper[b])
@@ -169,12 +169,13 @@ svdag_status tune_edits(svdag_ctx* ctx, const svdag_edit* edits, uint32_t n, svd
         sum[bucketOf[k]][formOf[k]] += ms * 1e3;
         cnt[bucketOf[k]][formOf[k]] += 1;
     }
-    // Persistent kernel for the buckets, from the smallest up, where it is faster.
+    // Building edits side by side, a block each, pays for the buckets, from the smallest up, where a block
+    // takes less than three chains one after another (launch_edits_at decides batch by batch).
     double threshold = 0;
     for (int b = 0; b < kBuckets - 1; ++b) {
         if (!cnt[b][0] || !cnt[b][1])
             break;
-        if (sum[b][1] / cnt[b][1] < sum[b][0] / cnt[b][0])
+        if (sum[b][1] / cnt[b][1] < 3.0 * sum[b][0] / cnt[b][0])
             threshold = upper[b];
         else
             break;

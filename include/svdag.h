@@ -57,9 +57,9 @@ typedef enum svdag_item_kind { SVDAG_KIND_NODE = 0, SVDAG_KIND_LEAF = 1 } svdag_
 /* Run every level's phases as launches of their own instead of the narrow levels (few items) of an edit
  * together in one block (for profiling single phases). */
 #define SVDAG_FLAG_PHASE_KERNELS 1u
-/* Run single edits whose intermediate SVO is estimated small (up to 16384 leaves) in the persistent kernel
- * (one CTA, block barriers between phases, one launch) instead of the chain of phase launches, and let
- * batches group such edits. svdag_autotune chooses the threshold by measurement. */
+/* Run single edits whose intermediate SVO is estimated small (up to 400 leaves) in the persistent kernel
+ * (one CTA, block barriers between phases, one launch) instead of the chain of phase launches where that
+ * is not slower, and let batches group edits of up to 16384 leaves. svdag_autotune chooses the threshold by measurement. */
 #define SVDAG_FLAG_PERSISTENT 2u
 
 typedef struct svdag_config {
@@ -516,17 +516,19 @@ svdag_status svdag_items_to_v3(const uint32_t* words, const uint64_t* level_word
  *    filled with it and searched for it, timed with CUDA events; the fastest pair is kept. The
  *    scratch tables' space is given back afterwards.
  *  - with an edit sample: the edits are applied in order (for real, each pushing its undo frame),
- *    alternately through the per-tool CUDA graph of the phase launches and through the persistent
- *    single-CTA kernel, each timed with CUDA events; the persistent kernel is kept for the size
- *    buckets of the estimated SVO leaves, from the smallest up, where it is faster.
+ *    alternately through the chain of phase launches and through the persistent single-CTA kernel,
+ *    each timed with CUDA events; batches group edits (one CTA each, side by side) of the size
+ *    buckets of the estimated SVO leaves, from the smallest up, where one CTA takes less than three
+ *    chains.
  * Synchronous; no other call may use the context meanwhile. */
 typedef struct svdag_tuning {
     uint32_t probe_lanes; /* lanes per key of the table kernels */
     uint32_t load_factor; /* items per bucket of tables sized from now on */
-    uint32_t persistent_leaves; /* edits estimated at or below this many SVO leaves use the persistent kernel (0 = none) */
+    uint32_t persistent_leaves; /* edits estimated at or below this many SVO leaves may be grouped in a batch
+                                   and, up to 400, run alone in the persistent kernel (0 = none) */
     uint32_t trials; /* measurements taken */
     double table_ns_per_key; /* best fill + search time per key of the key sample */
-    double graph_us_small; /* mean time of the sample's edits estimated below 4096 leaves: graph form */
+    double graph_us_small; /* mean time of the sample's edits estimated below 4096 leaves: chain of launches */
     double persistent_us_small; /* the same through the persistent kernel */
 } svdag_tuning;
 svdag_status svdag_autotune(svdag_ctx* ctx, const svdag_edit* edits, uint32_t n_edits, const uint32_t* keys_dev,
