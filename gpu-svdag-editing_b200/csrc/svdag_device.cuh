@@ -671,10 +671,9 @@ __device__ __forceinline__ uint32_t table_find(const Grp<G>& g, const DevDag& d,
             if (item_equals<G, LD_DEFAULT>(g, handle_ptr(d, item), key))
                 return item;
         }
-        if (next == kEnd || next == kLinking)
-            return kNone;
         if (!slab_ok(d, next)) {
-            set_status(d.ctl, SVDAG_ERR_CORRUPT);
+            if (next != kEnd && next != kLinking)
+                set_status(d.ctl, SVDAG_ERR_CORRUPT);
             return kNone;
         }
         slab = next;
