@@ -505,8 +505,8 @@ def run_serve(args):
                 "h2d_bytes_per_step": int(56 * len(ek) / args.steps),
                 "d2h_bytes_per_step": int((frame_d2h + 48 * len(ek)) / args.steps),
                 "detail": out["e2e"]},
-        "roofline": {"bound": "hbm", "kernel": "edit pipeline: one window of the stream as one batch (per-tool CUDA graphs of "
-                               "the phase kernels, small edits in the persistent kernel or in subtree groups)",
+        "roofline": {"bound": "hbm", "kernel": "edit pipeline: one window of the stream as one batch (a chain of launches "
+                               "per edit, small edits in subtree groups where that is faster)",
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": peak_kind, "traffic": None, "launch": bt},
         "trace_1080p": dict(out["trace"], bytes_per_ray_lower_bound=68 + 8 * levels,
@@ -514,8 +514,8 @@ def run_serve(args):
         "trace_c0": trace_c0,
         "batching": batching,
         "clocks": out["clocks"],
-        # launch calls of the timed served replay: one per batch (a CUDA-graph replay or one persistent
-        # kernel per run of small edits) and one per frame
+        # launch calls of the timed served replay: one per batch (a chain of kernels per edit or two
+        # kernels per group of small edits) and one per frame
         "gpu_launches": out["served"]["launches"] + fr.get("frames_whole", 0) + fr.get("frames_incremental", 0),
         "item_region_used_gb": out["used_gb"],
     }
@@ -875,7 +875,7 @@ def run_mode_c2(args):
                               persistent=args.persistent)
     build_s = time.perf_counter() - t0
     out = []
-    # capture every tool's graph before timing: a tiny edit of each kind far from the sequence, undone
+    # load every tool's kernels before timing: a tiny edit of each kind far from the sequence, undone
     for e in w.c2_edits(args.levels, terrain):
         tiny = w.make_edit(e.tool, 0, (3.0, 3.0, 3.0), 1.0, src=(3.0, 3.0, 3.0), dst=(5.0, 3.0, 3.0))
         dag.edit(tiny)
