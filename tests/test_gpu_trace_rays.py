@@ -1,6 +1,8 @@
 """Primary rays where the traversal's shortcuts could differ from the oracle: directions with zero and
 tiny components (their inverses are infinite or huge), cameras on node planes, inside, outside and far from
 the grid, at depths 4 to 17, images of odd and single-pixel sizes."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -60,3 +62,28 @@ def test_hits_equal_the_oracle(svdag_lib, oracle_mod, scene, view, size):
     assert np.array_equal(got["material"][hit], want["material"][hit])
     for f in ("position", "normal", "dpdu", "dpdv"):  # the same IEEE operations: the same floats
         assert np.array_equal(got[f], want[f], equal_nan=True), f
+
+
+@pytest.mark.parametrize("size", [(33, 4), (32, 4), (65, 8), (8, 65), (1, 1)])
+def test_shading_of_both_pixel_orders(svdag_lib, oracle_mod, scene, size):
+    """Images on both sides of the rule that gives a warp a row or a tile of pixels: sun visibility and
+    ambient occlusion equal the oracle's for every pixel, none is left out."""
+    import torch
+
+    levels, g, o = scene
+    n = float(1 << levels)
+    p = svdag_lib.get_trace_params([0.1 * n, 0.95 * n, 0.2 * n], [0.7 * n, 0.4 * n, 0.6 * n], *size)
+    po = oracle_mod.TraceParams()
+    for f in ("camera", "ray_min", "ray_ddx", "ray_ddy"):
+        getattr(po, f)[:] = list(getattr(p, f))
+    po.width, po.height = size
+    sh = svdag_lib.shade_params(levels, shadows=True, ao_samples=2, ao_ray_length=8.0)
+    so = oracle_mod.ShadeParams()
+    ctypes.memmove(ctypes.addressof(so), ctypes.addressof(sh), ctypes.sizeof(so))
+    tracer = svdag_lib.DAGTracer(*size)
+    tracer.resolve_paths(p, g)
+    colors, sun, ao = tracer.resolve_lighting(p, g, sh, want_surfaces=True)
+    torch.cuda.synchronize()
+    want = o.shade(po, so, o.trace(po))
+    assert np.array_equal(sun.cpu().numpy(), want[2])
+    assert np.array_equal(ao.cpu().numpy(), want[3])
