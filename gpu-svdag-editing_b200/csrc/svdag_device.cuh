@@ -620,25 +620,39 @@ __device__ __forceinline__ uint32_t append_slab(const Grp<G>& g, const DevDag& d
 {
     uint32_t* link = slab_ptr(d, slab) + 7;
     uint32_t next = 0;
+    if constexpr (G > 1 && G < 32) {
+        // Several groups share a warp: a wait of one holds up the others (2^24 adds with two lanes a key took
+        // 3.9 ms that way), so a group that still sees the end allocates, and the loser of a race gives its slab back.
+        if (g.lane == 0)
+            next = *reinterpret_cast<volatile uint32_t*>(link);
+        next = g.bcast(next, 0);
+        if (next == kEnd) {
+            const uint32_t fresh = alloc_slab<G>(g, d, k, t.recycle);
+            if (g.lane == 0 && fresh != kNone) {
+                next = atomicCAS(link, kEnd, fresh);
+                if (next != kEnd && t.recycle)
+                    push_free_chain(d, k - 2u, fresh, fresh, 1);
+            }
+            next = g.bcast(next, 0);
+            next = fresh == kNone ? kNone : next == kEnd ? fresh : next;
+        }
+        return next;
+    }
     if (g.lane == 0)
         next = atomicCAS(link, kEnd, kLinking);
     next = g.bcast(next, 0);
-    if (next == kEnd) {
-        const uint32_t fresh = alloc_slab<G>(g, d, k, t.recycle); // its header and body are visible to other SMs
+    const bool mine = next == kEnd;
+    if (mine) {
+        next = alloc_slab<G>(g, d, k, t.recycle); // its header and body are visible to other SMs
         if (g.lane == 0)
-            atomicExch(link, fresh == kNone ? kEnd : fresh);
-        g.sync();
-        return fresh;
-    }
-    if (g.lane == 0) {
-        for (uint32_t tries = 0; next == kLinking; ++tries) {
-            if (tries >= kLinkTries) {
-                set_status(d.ctl, SVDAG_ERR_TIMEOUT);
-                break;
-            }
+            atomicExch(link, next == kNone ? kEnd : next);
+    } else if (g.lane == 0) {
+        for (uint32_t tries = 0; next == kLinking && tries < kLinkTries; ++tries) {
             __nanosleep(64);
             next = *reinterpret_cast<volatile uint32_t*>(link);
         }
+        if (next == kLinking)
+            set_status(d.ctl, SVDAG_ERR_TIMEOUT);
         if (next == kLinking || next == kEnd) // timed out, or the allocation failed (and latched its error)
             next = kNone;
     }

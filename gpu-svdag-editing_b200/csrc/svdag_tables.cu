@@ -183,8 +183,18 @@ namespace {
 
 enum { OP_FIND = 0, OP_ADD = 1, OP_FIND_OR_INSERT = 2 };
 
+// Blocks an SM must hold, which caps the registers: lookups 32, adds 48 to 32, find-or-insert 64 to 40. All of
+// them wait for memory, so warps in flight count for more than a few spills of the rare paths (adds with
+// 32 lanes a key, 2^24 keys at 16 a bucket: 9.5 ms with 32 registers, 10.6 with 40); lower caps on one lane's add
+// cost 10 to 24 %.
 template <int G, int OP>
-__global__ void __launch_bounds__(256) k_table_op(DevDag d, DevTable t, const uint32_t* __restrict__ keys,
+constexpr int table_op_blocks()
+{
+    return OP == OP_FIND ? 8 : OP == OP_ADD ? (G == 1 ? 5 : G < 16 ? 6 : 8) : (G < 4 ? 4 : 6);
+}
+
+template <int G, int OP>
+__global__ void __launch_bounds__(256, table_op_blocks<G, OP>()) k_table_op(DevDag d, DevTable t, const uint32_t* __restrict__ keys,
     const uint32_t* __restrict__ offsets, uint32_t n, unsigned long long totalWords, const uint32_t* __restrict__ reps,
     uint32_t* __restrict__ out)
 {
