@@ -1394,17 +1394,20 @@ union NarrowShared {
     uint32_t leaves[kBlockThreads / 8 * leaf_shared_words<SVDAG_TOOL_COPY>()]; // the leaf phase of a block's edit
 };
 
-// GPU-clock stamps at the phase barriers (svdag_last_edit_phase_times).
+// GPU-clock stamps at the phase barriers of an edit that one block runs (svdag_last_edit_phase_times). An
+// edit's chain of launches takes none and leaves the last ones as they are: its kernels pass kNoStamps.
+constexpr uint32_t kNoStamps = 64;
 __device__ __forceinline__ void stamp(const DevDag& d, uint32_t& k)
 {
-    if (!d.solo && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (k < kNoStamps && !d.solo && blockIdx.x == 0 && threadIdx.x == 0) {
         unsigned long long t;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-        if (k < 64)
-            d.ctl->phaseTimes[k] = t;
+        d.ctl->phaseTimes[k] = t;
         d.ctl->phaseCount = ++k;
     }
 }
+static_assert(kNoStamps == sizeof(Control::phaseTimes) / sizeof(Control::phaseTimes[0]) && 2 * kMaxLevels + 4 < kNoStamps,
+    "an edit's stamps fit");
 
 // Top-down phases of the levels from the edit's first one while they are below `endLevel` and narrow,
 // in one block (all threads call); returns the first level left. Its work items are in scratch, as
@@ -1734,7 +1737,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_edit_top(DevDag d, const _
     __syncthreads();
     ph_edit_begin(d, e, scratch);
     __syncthreads();
-    uint32_t k = 64; // no stamps
+    uint32_t k = kNoStamps;
     if (narrow_build<TOOL>(d, e, endLevel, scratch, scratchBytes, sh, k) < endLevel && threadIdx.x == 0) { // ruled out by the caller's bounds
         set_status(d.ctl, SVDAG_ERR_CORRUPT);
         d.edit->overflow = 1;
@@ -1776,7 +1779,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_edit_bottom(DevDag d, uint
 {
     __shared__ NarrowShared sh;
     chain_wait();
-    uint32_t k = 64, root = kNone; // no stamps
+    uint32_t k = kNoStamps, root = kNone;
     if (endLevel > startLevel)
         root = narrow_merge<false>(d, endLevel - 1u, scratch, sh, k);
     else if (merge_live(d))
