@@ -609,44 +609,73 @@ __device__ __forceinline__ uint32_t alloc_slab(const Grp<G>& g, const DevDag& d,
     return id;
 }
 
-// The slab after `slab` in its chain, appended when the chain ends there. The thread that turns the
-// end mark into kLinking allocates; the others wait for the link it publishes (bounded, then
-// SVDAG_ERR_TIMEOUT). A full bucket so costs one slab and one trip to the allocator however many
-// threads find it full at once: when every one of them allocated and all but one gave their slab
-// back, a tile of a depth-13 scene build spent 22 ms of one merge launch on the free list's head word.
-// kNone when a region is full (SVDAG_ERR_OOM) or the wait ran out.
+// An overflow slab that a group of 2 to 16 lanes allocated but did not get to link: the group's next append
+// of that size class links it. Other groups hold none.
+struct Spare {
+    uint32_t slab = kNone;
+    uint32_t k = 0;
+};
+
+// Gives an unused spare back: a level table's goes on its class's free list; other tables' spares
+// stay allocated (their space comes back when the bump pointers are rewound or never).
 template <int G>
-__device__ __forceinline__ uint32_t append_slab(const Grp<G>& g, const DevDag& d, const DevTable& t, uint32_t slab, uint32_t k)
+__device__ __forceinline__ void release_spare(const Grp<G>& g, const DevDag& d, uint32_t recycle, Spare& spare)
+{
+    if (spare.slab != kNone && recycle && g.lane == 0)
+        push_free_chain(d, spare.k - 2u, spare.slab, spare.slab, 1);
+    spare.slab = kNone;
+}
+
+// The slab after `slab` in its chain, appended when the chain ends there; kNone when a region is full
+// (SVDAG_ERR_OOM) or a wait ran out (SVDAG_ERR_TIMEOUT).
+// One lane a key, and 32: the thread that turns the end mark into kLinking allocates; the others wait for
+// the link it publishes (bounded). A full bucket so costs one slab and one trip to the allocator however
+// many threads find it full at once: when every one of them allocated and all but one gave their slab
+// back, a tile of a depth-13 scene build spent 22 ms of one merge launch on the free list's head word.
+// 2 to 16 lanes: a wait of one group holds up the others of its warp (2^24 adds with two lanes a key took
+// 3.9 ms that way, 1.3 this way), so a group that still sees the end allocates; the loser of a race keeps its slab
+// for its next append of that size class, so keys of one class take at most one slab a group more than their
+// chains hold. `recycle`: the table's.
+template <int G>
+__device__ __forceinline__ uint32_t append_slab(const Grp<G>& g, const DevDag& d, uint32_t recycle, uint32_t slab, uint32_t k,
+    Spare& spare)
 {
     uint32_t* link = slab_ptr(d, slab) + 7;
     uint32_t next = 0;
+    bool mine = false;
     if constexpr (G > 1 && G < 32) {
-        // Several groups share a warp: a wait of one holds up the others (2^24 adds with two lanes a key took
-        // 3.9 ms that way), so a group that still sees the end allocates, and the loser of a race gives its slab back.
         if (g.lane == 0)
             next = *reinterpret_cast<volatile uint32_t*>(link);
         next = g.bcast(next, 0);
         if (next == kEnd) {
-            const uint32_t fresh = alloc_slab<G>(g, d, k, t.recycle);
-            if (g.lane == 0 && fresh != kNone) {
-                next = atomicCAS(link, kEnd, fresh);
-                if (next != kEnd && t.recycle)
-                    push_free_chain(d, k - 2u, fresh, fresh, 1);
+            if (spare.slab == kNone || spare.k != k) { // a spare of another size class goes first
+                release_spare<G>(g, d, recycle, spare);
+                spare.slab = alloc_slab<G>(g, d, k, recycle);
+                spare.k = k;
             }
+            if (spare.slab == kNone)
+                return kNone;
+            if (g.lane == 0)
+                next = atomicCAS(link, kEnd, spare.slab);
             next = g.bcast(next, 0);
-            next = fresh == kNone ? kNone : next == kEnd ? fresh : next;
+            if (next == kEnd) {
+                mine = true;
+                next = spare.slab;
+                spare.slab = kNone;
+            }
         }
-        return next;
-    }
-    if (g.lane == 0)
-        next = atomicCAS(link, kEnd, kLinking);
-    next = g.bcast(next, 0);
-    const bool mine = next == kEnd;
-    if (mine) {
-        next = alloc_slab<G>(g, d, k, t.recycle); // its header and body are visible to other SMs
+    } else {
         if (g.lane == 0)
-            atomicExch(link, next == kNone ? kEnd : next);
-    } else if (g.lane == 0) {
+            next = atomicCAS(link, kEnd, kLinking);
+        next = g.bcast(next, 0);
+        if (next == kEnd) {
+            mine = true;
+            next = alloc_slab<G>(g, d, k, recycle); // its header and body are visible to other SMs
+            if (g.lane == 0)
+                atomicExch(link, next == kNone ? kEnd : next);
+        }
+    }
+    if (!mine && g.lane == 0) {
         for (uint32_t tries = 0; next == kLinking && tries < kLinkTries; ++tries) {
             __nanosleep(64);
             next = *reinterpret_cast<volatile uint32_t*>(link);
@@ -739,7 +768,7 @@ __device__ __forceinline__ uint32_t claim_in_slab(const Grp<G>& g, const DevDag&
 // Unconditional insert (CompactAccelerationHashTable::addAsWarp, compact_acceleration_hash_table.h:63-121):
 // the key gets a fresh slot even when an equal key is stored already.
 template <int G>
-__device__ __forceinline__ uint32_t table_add(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key)
+__device__ __forceinline__ uint32_t table_add(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key, Spare& spare)
 {
     const uint32_t cls = key.n - 2u;
     if (key.n < 2u || key.n > 10u || t.numBuckets[cls] == 0) {
@@ -758,7 +787,7 @@ __device__ __forceinline__ uint32_t table_add(const Grp<G>& g, const DevDag& d, 
             return item;
         }
         if (next == kEnd || next == kLinking) {
-            next = append_slab<G>(g, d, t, slab, key.n);
+            next = append_slab<G>(g, d, t.recycle, slab, key.n, spare);
             if (next == kNone)
                 return kNone;
         }
@@ -847,7 +876,8 @@ __device__ __forceinline__ uint32_t table_probe(const Grp<G>& g, const DevDag& d
 enum : int { kPublish = 0, kQuiet = 1, kSole = 2 };
 
 template <int G, int HOW = kPublish>
-__device__ __forceinline__ uint32_t table_insert_probed(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key, Probed<G>& at)
+__device__ __forceinline__ uint32_t table_insert_probed(const Grp<G>& g, const DevDag& d, uint32_t recycle, const Key<G>& key, Probed<G>& at,
+    Spare& spare)
 {
     const uint32_t tag = tag_of(key.hb);
     uint32_t slab = at.slab, empty = at.empty, body = at.body;
@@ -884,7 +914,7 @@ __device__ __forceinline__ uint32_t table_insert_probed(const Grp<G>& g, const D
         if (empty)
             continue; // a slot was freed up meanwhile (cannot happen during edits, kept for safety)
         if (next == kEnd || next == kLinking) {
-            next = append_slab<G>(g, d, t, slab, key.n);
+            next = append_slab<G>(g, d, recycle, slab, key.n, spare);
             if (next == kNone)
                 return kNone;
         }
@@ -912,7 +942,8 @@ enum : int { kInsertLaunch = 0, kInsertShared = 1 };
 // two equal keys finds the first's published item. A holder only probes and inserts into its own chain,
 // so no lock waits on another; the wait for a lock is bounded and ends with SVDAG_ERR_TIMEOUT.
 template <int G, int MODE = kInsertLaunch>
-__device__ __forceinline__ uint32_t table_find_or_insert(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key, bool& inserted)
+__device__ __forceinline__ uint32_t table_find_or_insert(const Grp<G>& g, const DevDag& d, const DevTable& t, const Key<G>& key, Spare& spare,
+    bool& inserted)
 {
     inserted = false;
     Probed<G> at;
@@ -937,14 +968,14 @@ __device__ __forceinline__ uint32_t table_find_or_insert(const Grp<G>& g, const 
         __threadfence(); // acquire: the previous holder's item and tag are visible
         h = table_probe<G>(g, d, t, key, at, ok);
         if (h == kNone && ok) {
-            h = table_insert_probed<G>(g, d, t, key, at);
+            h = table_insert_probed<G>(g, d, t.recycle, key, at, spare);
             inserted = h != kNone;
         }
         __threadfence(); // release: this holder's item and tag are visible before the lock is free
         atomicExch(lock, 0u);
         return h;
     } else {
-        h = table_insert_probed<G>(g, d, t, key, at);
+        h = table_insert_probed<G>(g, d, t.recycle, key, at, spare);
         inserted = h != kNone;
         return h;
     }

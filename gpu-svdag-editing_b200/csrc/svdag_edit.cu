@@ -1153,7 +1153,8 @@ __device__ uint32_t merge_single(const DevDag& d, uint32_t level, uint32_t* w, c
     E.repCount[level] = 1;
     const DevTable& t = d.ctl->tables[level];
     bool ins = false;
-    const uint32_t h = table_find_or_insert<1, MODE>(g, d, t, key, ins);
+    Spare none; // one lane a key holds no spare
+    const uint32_t h = table_find_or_insert<1, MODE>(g, d, t, key, none, ins);
     added += ins ? 1u : 0u;
     return h;
 }
@@ -1185,6 +1186,7 @@ __device__ void ph_merge_level(const DevDag& d, uint32_t level, char* scratch)
     uint32_t* items = reinterpret_cast<uint32_t*>(scratch + E.offN[level]);
     const DevTable& t = d.ctl->tables[level]; // in memory: a copy indexed by size class would live on the stack
     Grp<1> g;
+    Spare none; // one lane a key holds no spare
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t full = 0, reps = 0, added = 0;
     for (uint32_t base = ph_block(d) * blockDim.x; base < n; base += ph_grid(d) * blockDim.x) { // whole warps
@@ -1261,7 +1263,7 @@ __device__ void ph_merge_level(const DevDag& d, uint32_t level, char* scratch)
             if (r == i) {
                 ++reps;
                 bool ins = false;
-                handle[i] = table_find_or_insert<1, SHARED ? kInsertShared : kInsertLaunch>(g, d, t, key, ins);
+                handle[i] = table_find_or_insert<1, SHARED ? kInsertShared : kInsertLaunch>(g, d, t, key, none, ins);
                 added += ins ? 1u : 0u;
             }
         }
@@ -1292,6 +1294,7 @@ __device__ void ph_insert_level(const DevDag& d, const DevTable& t, uint32_t lev
     const uint32_t* items = reinterpret_cast<const uint32_t*>(scratch + E.offN[level]);
     Grp<G> g;
     const uint32_t groupsPerBlock = blockDim.x / G;
+    Spare spare;
     uint32_t added = 0;
     for (uint32_t i = ph_block(d) * groupsPerBlock + threadIdx.x / G; i < n; i += ph_grid(d) * groupsPerBlock) {
         if (rep[i] != i)
@@ -1299,12 +1302,13 @@ __device__ void ph_insert_level(const DevDag& d, const DevTable& t, uint32_t lev
         Key<G> key;
         load_key<G>(g, items + (size_t)i * kItemStride, kItemStride, t.kind, key);
         bool ins = false;
-        const uint32_t h = table_find_or_insert<G>(g, d, t, key, ins);
+        const uint32_t h = table_find_or_insert<G>(g, d, t, key, spare, ins);
         if (g.lane == 0) {
             handle[i] = h;
             added += ins ? 1u : 0u;
         }
     }
+    release_spare<G>(g, d, t.recycle, spare);
     if (added)
         atomicAdd(&E.added, (unsigned long long)added);
 }
@@ -1564,6 +1568,7 @@ __device__ uint32_t narrow_merge(const DevDag& d, uint32_t fromLevel, char* scra
     auto& M = sh.merge;
     const uint32_t LL = d.leafLevel, tid = threadIdx.x, startLevel = E.startLevel, builder = E.builder;
     Grp<1> g;
+    Spare none; // one lane a key holds no spare
     for (uint32_t k = tid; k < sizeof(M.tables) / 4; k += blockDim.x)
         reinterpret_cast<uint32_t*>(M.tables)[k] = reinterpret_cast<const uint32_t*>(d.ctl->tables)[k];
     for (uint32_t l = tid; l < kMaxLevels; l += blockDim.x) {
@@ -1650,14 +1655,14 @@ __device__ uint32_t narrow_merge(const DevDag& d, uint32_t fromLevel, char* scra
             if (n > 1)
                 __syncthreads(); // the duplicate search is over before its table is cleared below
             if (mine)
-                h = table_find_or_insert<1, kInsertShared>(g, d, M.tables[level], key, inserted);
+                h = table_find_or_insert<1, kInsertShared>(g, d, M.tables[level], key, none, inserted);
         } else if (n == 1) {
             if (mine) {
                 Probed<1> at;
                 bool ok;
                 h = table_probe<1>(g, d, M.tables[level], key, at, ok);
                 if (h == kNone && ok) {
-                    h = table_insert_probed<1, kSole>(g, d, M.tables[level], key, at);
+                    h = table_insert_probed<1, kSole>(g, d, M.tables[level].recycle, key, at, none);
                     inserted = h != kNone;
                 }
             }
@@ -1668,7 +1673,7 @@ __device__ uint32_t narrow_merge(const DevDag& d, uint32_t fromLevel, char* scra
                 h = table_probe<1>(g, d, M.tables[level], key, at, ok);
             __syncthreads(); // lookups are over: inserts need not hide their unfinished items
             if (mine && h == kNone && ok) {
-                h = table_insert_probed<1, kQuiet>(g, d, M.tables[level], key, at);
+                h = table_insert_probed<1, kQuiet>(g, d, M.tables[level].recycle, key, at, none);
                 inserted = h != kNone;
             }
         }

@@ -106,7 +106,8 @@ __global__ void k_insert_canonical(DevDag d, DevTable t, uint32_t level)
         }
         hash_words(key.w, key.n, key.ha, key.hb);
         bool inserted;
-        d.ctl->fullyFilled[level][m] = table_find_or_insert<1>(g, d, t, key, inserted);
+        Spare none; // one lane a key holds no spare
+        d.ctl->fullyFilled[level][m] = table_find_or_insert<1>(g, d, t, key, none, inserted);
     }
 }
 
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(256, table_op_blocks<G, OP>()) k_table_op(DevD
     Grp<G> g;
     const uint32_t groupsPerBlock = blockDim.x / G;
     const unsigned long long stride = (unsigned long long)gridDim.x * groupsPerBlock;
+    Spare spare;
     for (unsigned long long i = blockIdx.x * groupsPerBlock + threadIdx.x / G; i < n; i += stride) {
         if (reps && reps[i] != i)
             continue;
@@ -217,14 +219,15 @@ __global__ void __launch_bounds__(256, table_op_blocks<G, OP>()) k_table_op(DevD
         if constexpr (OP == OP_FIND) {
             h = table_find<G>(g, d, t, key);
         } else if constexpr (OP == OP_ADD) {
-            h = table_add<G>(g, d, t, key);
+            h = table_add<G>(g, d, t, key, spare);
         } else {
             bool ins;
-            h = table_find_or_insert<G>(g, d, t, key, ins);
+            h = table_find_or_insert<G>(g, d, t, key, spare, ins);
         }
         if (g.lane == 0)
             out[i] = h;
     }
+    release_spare<G>(g, d, t.recycle, spare);
 }
 
 // Batch dedup into an open-addressing scratch table of 64-bit entries (tag hash << 32 | index+1).
