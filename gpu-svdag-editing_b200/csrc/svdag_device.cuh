@@ -626,6 +626,22 @@ __device__ __forceinline__ void release_spare(const Grp<G>& g, const DevDag& d, 
     spare.slab = kNone;
 }
 
+// The slab that another thread appends: `next` is what the link held (bounded, then SVDAG_ERR_TIMEOUT). kNone when
+// the wait ran out or that thread's allocation failed (and latched its error). Out of line with several lanes a key,
+// whose loops over keys it slows where nothing waits: 2^24 adds at 96 a bucket 4.24 ms inlined and 3.19 so with 4 lanes,
+// 5.43 and 4.15 with 8.
+__device__ __forceinline__ uint32_t wait_link(Control* ctl, uint32_t* link, uint32_t next)
+{
+    for (uint32_t tries = 0; next == kLinking && tries < kLinkTries; ++tries) {
+        __nanosleep(64);
+        next = *reinterpret_cast<volatile uint32_t*>(link);
+    }
+    if (next == kLinking)
+        set_status(ctl, SVDAG_ERR_TIMEOUT);
+    return next == kLinking || next == kEnd ? kNone : next;
+}
+static __device__ __noinline__ uint32_t wait_link_call(Control* ctl, uint32_t* link, uint32_t next) { return wait_link(ctl, link, next); }
+
 // The slab after `slab` in its chain, appended when the chain ends there; kNone when a region is full
 // (SVDAG_ERR_OOM) or a wait ran out (SVDAG_ERR_TIMEOUT).
 // One lane a key, and 32: the thread that turns the end mark into kLinking allocates; the others wait for
@@ -675,16 +691,10 @@ __device__ __forceinline__ uint32_t append_slab_inline(const Grp<G>& g, const De
                 atomicExch(link, next == kNone ? kEnd : next);
         }
     }
-    if (!mine && g.lane == 0) {
-        for (uint32_t tries = 0; next == kLinking && tries < kLinkTries; ++tries) {
-            __nanosleep(64);
-            next = *reinterpret_cast<volatile uint32_t*>(link);
-        }
-        if (next == kLinking)
-            set_status(d.ctl, SVDAG_ERR_TIMEOUT);
-        if (next == kLinking || next == kEnd) // timed out, or the allocation failed (and latched its error)
-            next = kNone;
-    }
+    if (mine || (next != kLinking && next != kEnd))
+        return next;
+    if (g.lane == 0)
+        next = G > 1 ? wait_link_call(d.ctl, link, next) : wait_link(d.ctl, link, next);
     return g.bcast(next, 0);
 }
 
