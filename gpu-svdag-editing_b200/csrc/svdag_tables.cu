@@ -185,13 +185,14 @@ namespace {
 enum { OP_FIND = 0, OP_ADD = 1, OP_FIND_OR_INSERT = 2 };
 
 // Blocks an SM must hold, which caps the registers: lookups 32, adds 48 to 32, find-or-insert 64 to 40. All of
-// them wait for memory, so warps in flight count for more than a few spills of the rare paths (adds with
-// 32 lanes a key, 2^24 keys at 16 a bucket: 9.5 ms with 32 registers, 10.6 with 40); lower caps on one lane's add
-// cost 10 to 24 %.
+// them wait for memory, so warps in flight count for more than a few spills of the rare paths (adds of 2^21 keys
+// at 16 a bucket with 32 lanes a key: 617 us with 32 registers, 866 with 40; with 16: 413 and 550); lower caps on one
+// lane's add cost 10 to 24 %. A lookup with 32 lanes has no cap (2^22 keys at 96 a bucket: 2329 us without, 2560
+// with).
 template <int G, int OP>
 constexpr int table_op_blocks()
 {
-    return OP == OP_FIND ? 8 : OP == OP_ADD ? (G == 1 ? 5 : G < 16 ? 6 : 8) : (G < 4 ? 4 : 6);
+    return OP == OP_FIND ? (G == 32 ? 1 : 8) : OP == OP_ADD ? (G == 1 ? 5 : G < 16 ? 6 : 8) : (G < 4 ? 4 : 6);
 }
 
 template <int G, int OP>
