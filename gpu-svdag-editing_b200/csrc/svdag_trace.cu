@@ -144,7 +144,6 @@ __device__ __forceinline__ bool ray_meets_box(const RayF& r, const float* b)
 // intersect_ray, tracer.cu:186-273: the first voxel on the ray and its material; leaves the coordinates as they
 // are when there is none. Stack in shared memory, [level][thread] so that a warp's accesses hit distinct
 // banks. Bound by the integer and compare pipe (75 % busy).
-template <bool TAME>
 __device__ __forceinline__ void first_hit(const DevDag& d, uint32_t root, const RayF& r, uint32_t (*sIndex)[256], uint32_t (*sMasks)[256],
     const uint8_t* sNext, uint32_t tix, uint32_t& px, uint32_t& py, uint32_t& pz, uint32_t& material)
 {
@@ -153,7 +152,7 @@ __device__ __forceinline__ void first_hit(const DevDag& d, uint32_t root, const 
     uint32_t level = 0, X = kCoordBias, Y = kCoordBias, Z = kCoordBias, leafLo = 0, leafHi = 0;
     uint32_t node = root;
     uint32_t children = checked_item(d, last, root)[0] & 0xFFu;
-    uint32_t visit = children & intersection_mask<TAME>(true, levels, X, Y, Z, r);
+    uint32_t visit = children & intersection_mask<false>(true, levels, X, Y, Z, r);
     // Bit l of `live`: the stack entry of level l still has children to visit. Ascending to the
     // deepest such level below the current one is what the reference's pop loop does one level
     // at a time (entries in between have nothing left); here it is one bit scan.
@@ -211,7 +210,7 @@ __device__ __forceinline__ void first_hit(const DevDag& d, uint32_t root, const 
         } else { // get_second_child_mask, base_dag.h:53-58
             children = (((child & 4u) ? leafHi : leafLo) >> ((child & 3u) * 8u)) & 0xFFu;
         }
-        visit = children & intersection_mask<TAME>(false, levels - level, X, Y, Z, r);
+        visit = children & intersection_mask<false>(false, levels - level, X, Y, Z, r);
     }
 }
 
@@ -269,10 +268,9 @@ __global__ void __launch_bounds__(256) k_trace(DevDag d, svdag_trace_params p, s
     uint32_t px = 0, py = 0, pz = 0, material = 0xFFFFFFFFu;
     const uint32_t root = rootPtr ? *rootPtr : d.ctl->root;
     if (root != kNone) {
-        if (ray_tame(r))
-            first_hit<true>(d, root, r, sIndex, sMasks, sNext, tix, px, py, pz, material);
-        else
-            first_hit<false>(d, root, r, sIndex, sMasks, sNext, tix, px, py, pz, material);
+        const uint32_t lanes = __activemask(); // as in any_hit
+        first_hit(d, root, r, sIndex, sMasks, sNext, tix, px, py, pz, material);
+        __syncwarp(lanes);
     }
     if (px == 0 && py == 0 && pz == 0)
         material = 0xFFFFFFFFu; // a miss has no material (Path::is_null, path.h:61-64)
