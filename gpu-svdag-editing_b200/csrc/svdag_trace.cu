@@ -30,9 +30,14 @@ __device__ __forceinline__ float pow2_float(uint32_t e) { return __uint_as_float
 constexpr uint32_t kCoordBias = 0x4B000000u;
 __device__ __forceinline__ float coord_float(uint32_t biased) { return __uint_as_float(biased) - 8388608.0f; }
 
-// A ray all of whose inverse direction components are at most 1e30 in magnitude: every product and sum of its
-// intersection tests is finite, so no NaN reaches a comparison.
-__device__ __forceinline__ bool ray_tame(const RayF& r) { return fabsf(r.ix) <= 1e30f && fabsf(r.iy) <= 1e30f && fabsf(r.iz) <= 1e30f; }
+// A ray all of whose inverse direction components are at most 1e30 in magnitude and whose origin has no NaN (nor
+// infinities of both signs): every product and sum of its intersection tests is finite, or an infinity that meets no
+// opposite one, so no NaN reaches a comparison.
+__device__ __forceinline__ bool ray_tame(const RayF& r)
+{
+    const float origin = (r.ox + r.oy) + r.oz;
+    return fabsf(r.ix) <= 1e30f && fabsf(r.iy) <= 1e30f && fabsf(r.iz) <= 1e30f && origin == origin;
+}
 
 // compute_intersection_mask, tracer.cu:56-173, of the node of size 2^shift with the biased corner (X, Y, Z)
 // (device max/min of two floats are fmaxf/fminf; the vector max/min of cuda_math.h are the ternary forms,
