@@ -159,8 +159,9 @@ __device__ __forceinline__ void set_status(Control* ctl, uint32_t code)
 }
 
 // Every handle read from memory is checked before it is dereferenced: a bad handle (which only a
-// bug could produce) latches SVDAG_ERR_CORRUPT and reads a zero item instead of faulting.
-__device__ const uint32_t kZeroItem[16] = {};
+// bug could produce) latches SVDAG_ERR_CORRUPT and reads a zero item instead of faulting. Items are read in
+// words of up to 16 bytes, so it is aligned as they are.
+__device__ const __align__(16) uint32_t kZeroItem[16] = {};
 __device__ __forceinline__ bool handle_ok(const DevDag& d, uint32_t h)
 {
     return (unsigned long long)kUnitWords * h + 16ull <= d.itemWords;
