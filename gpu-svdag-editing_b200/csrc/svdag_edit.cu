@@ -2564,9 +2564,9 @@ svdag_status reset_dag(svdag_ctx* ctx, cudaStream_t s)
 // fully-filled bits everywhere, my_gpu_hash_dag_factory.cpp:350-353) and each level table sized from
 // the exact number of distinct items of that level (the reference resizes with setLoadFactor
 // afterwards, my_gpu_hash_dag.cu:139-155).
-svdag_status build_scene_untiled(svdag_ctx* ctx, const DevEditor& ed, cudaStream_t s)
+// `least`: the level tables' minimum; `sized` tells whether the build came to a table.
+static svdag_status build_scene_untiled_into(svdag_ctx* ctx, const DevEditor& ed, uint32_t least, bool& sized, cudaStream_t s)
 {
-    SVDAG_TRY(reset_dag(ctx, s));
     const DevDag d = ctx->dag();
     const uint32_t LL = d.leafLevel;
     SVDAG_TRY(launch_chained(k_edit_top<kToolTerrain>, 1, kBlockThreads, false, s, d, ed, ed.startLevel, ctx->scratch, ctx->scratchBytes));
@@ -2593,7 +2593,8 @@ svdag_status build_scene_untiled(svdag_ctx* ctx, const DevEditor& ed, cudaStream
             buckets[c] = (uint32_t)std::max<unsigned long long>(1, (items + ctx->loadFactor - 1) / ctx->loadFactor);
         }
         svdag_table& t = ctx->levelTables[level];
-        SVDAG_TRY(alloc_level_table(ctx, &t, level == (int)LL ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets, s));
+        sized = true;
+        SVDAG_TRY(alloc_level_table(ctx, &t, level == (int)LL ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets, least, s));
         t.level = level;
         SVDAG_TRY(upload_tables(ctx, s));
         SVDAG_TRY(insert_canonical(ctx, (uint32_t)level, s));
@@ -2602,6 +2603,20 @@ svdag_status build_scene_untiled(svdag_ctx* ctx, const DevEditor& ed, cudaStream
     SVDAG_TRY(launch_chained(k_edit_bottom, 1, kBlockThreads, true, s, d, ed.startLevel, ed.startLevel, ed.builder, ed.tileOut, (EditRecord*)nullptr,
         ctx->scratch));
     return read_status(ctx, s);
+}
+
+// The sizes that the scene wants are known level by level only, so the minimum takes its share of the whole region.
+svdag_status build_scene_untiled(svdag_ctx* ctx, const DevEditor& ed, cudaStream_t s)
+{
+    SVDAG_TRY(reset_dag(ctx, s));
+    uint32_t least = 0;
+    SVDAG_TRY(level_table_minimum(ctx, TableSpace {}, &least, s));
+    bool sized = false;
+    const svdag_status st = build_scene_untiled_into(ctx, ed, least, sized, s);
+    if (st != SVDAG_ERR_OOM || !sized || !least)
+        return st;
+    SVDAG_TRY(reset_dag(ctx, s));
+    return build_scene_untiled_into(ctx, ed, 0, sized, s);
 }
 
 // Tiles of a scene: every tile is a builder edit of the subtree under one node, all tiles of a call

@@ -88,7 +88,19 @@ svdag_status insert_canonical(svdag_ctx* ctx, uint32_t level, cudaStream_t s);
 svdag_status upload_tables(svdag_ctx* ctx, cudaStream_t s);
 svdag_status read_status(svdag_ctx* ctx, cudaStream_t s);
 void reset_level_tables(svdag_ctx* ctx);
-svdag_status alloc_level_table(svdag_ctx* ctx, svdag_table* t, uint32_t kind, const uint32_t* bucketsPerClass, cudaStream_t s);
+// Space of the bucket arrays of tables: words of the item region, headers of the header region.
+struct TableSpace {
+    unsigned long long words = 0, headers = 0;
+    void add(const uint32_t* bucketsPerClass)
+    {
+        for (uint32_t c = 0; c < kNumClasses; ++c) {
+            words += (unsigned long long)bucketsPerClass[c] * body_words(c + 2);
+            headers += bucketsPerClass[c];
+        }
+    }
+};
+svdag_status level_table_minimum(svdag_ctx* ctx, const TableSpace& wanted, uint32_t* least, cudaStream_t s);
+svdag_status alloc_level_table(svdag_ctx* ctx, svdag_table* t, uint32_t kind, const uint32_t* bucketsPerClass, uint32_t least, cudaStream_t s);
 // Find-or-insert of keys that are pairwise distinct (no batch dedup) into a level table.
 svdag_status find_or_insert_distinct(svdag_ctx* ctx, uint32_t level, const uint32_t* keys, const uint32_t* offsets, uint32_t n,
     unsigned long long totalWords, uint32_t* out, cudaStream_t s);

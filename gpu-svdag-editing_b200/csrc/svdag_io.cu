@@ -93,14 +93,20 @@ svdag_status insert_level(svdag_ctx* ctx, uint32_t level, const std::vector<uint
     return read_status(ctx, s);
 }
 
+// Buckets of a size class of a level table for `items` items and the canonical ones.
+static uint32_t table_buckets(const svdag_ctx* ctx, unsigned long long items)
+{
+    return (uint32_t)std::max<unsigned long long>(1, (items + SVDAG_NUM_MATERIALS + ctx->loadFactor - 1) / ctx->loadFactor);
+}
+
 // Replaces the context's DAG by a snapshot (already validated), bottom-up: the items of a level are
 // deduplicated on the host, the level table is sized for them exactly (as a scene build sizes it),
 // and its parents' child ordinals are rewritten to the handles the table returned.
-svdag_status load_snapshot(svdag_ctx* ctx, const uint32_t* words, const uint64_t* levelWords, const uint64_t* levelItems,
-    const std::vector<std::vector<uint64_t>>& offsets, cudaStream_t s)
+// `least`: the level tables' minimum.
+static svdag_status load_snapshot_into(svdag_ctx* ctx, const uint32_t* words, const uint64_t* levelWords, const uint64_t* levelItems,
+    const std::vector<std::vector<uint64_t>>& offsets, uint32_t least, cudaStream_t s)
 {
     const uint32_t LL = ctx->cfg.levels - 2;
-    SVDAG_TRY(reset_dag(ctx, s));
     std::vector<uint64_t> base(LL + 2, 0);
     for (uint32_t l = 0; l <= LL; ++l)
         base[l + 1] = base[l] + levelWords[l];
@@ -137,9 +143,9 @@ svdag_status load_snapshot(svdag_ctx* ctx, const uint32_t* words, const uint64_t
         }
         uint32_t buckets[kNumClasses];
         for (uint32_t c = 0; c < kNumClasses; ++c)
-            buckets[c] = (uint32_t)std::max<unsigned long long>(1, (perClass[c] + SVDAG_NUM_MATERIALS + ctx->loadFactor - 1) / ctx->loadFactor);
+            buckets[c] = table_buckets(ctx, perClass[c]);
         svdag_table& t = ctx->levelTables[level];
-        SVDAG_TRY(alloc_level_table(ctx, &t, leaf ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets, s));
+        SVDAG_TRY(alloc_level_table(ctx, &t, leaf ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets, least, s));
         t.level = (uint32_t)level;
         SVDAG_TRY(upload_tables(ctx, s));
         SVDAG_TRY(insert_canonical(ctx, (uint32_t)level, s));
@@ -153,6 +159,32 @@ svdag_status load_snapshot(svdag_ctx* ctx, const uint32_t* words, const uint64_t
     SVDAG_CUDA(cudaMemcpyAsync(&ctx->ctl->root, &root, sizeof(root), cudaMemcpyHostToDevice, s));
     SVDAG_CUDA(cudaStreamSynchronize(s));
     return read_status(ctx, s);
+}
+
+svdag_status load_snapshot(svdag_ctx* ctx, const uint32_t* words, const uint64_t* levelWords, const uint64_t* levelItems,
+    const std::vector<std::vector<uint64_t>>& offsets, cudaStream_t s)
+{
+    const uint32_t LL = ctx->cfg.levels - 2;
+    TableSpace wanted; // of the snapshot's items, equal ones counted apart
+    uint64_t base = 0;
+    for (uint32_t level = 0; level <= LL; ++level) {
+        unsigned long long perClass[kNumClasses] = {};
+        for (const uint64_t off : offsets[level])
+            perClass[item_words(level == LL, words + base + off, levelWords[level] - off) - 2]++;
+        uint32_t buckets[kNumClasses];
+        for (uint32_t c = 0; c < kNumClasses; ++c)
+            buckets[c] = table_buckets(ctx, perClass[c]);
+        wanted.add(buckets);
+        base += levelWords[level];
+    }
+    SVDAG_TRY(reset_dag(ctx, s));
+    uint32_t least = 0;
+    SVDAG_TRY(level_table_minimum(ctx, wanted, &least, s));
+    const svdag_status st = load_snapshot_into(ctx, words, levelWords, levelItems, offsets, least, s);
+    if (st != SVDAG_ERR_OOM || !least)
+        return st;
+    SVDAG_TRY(reset_dag(ctx, s));
+    return load_snapshot_into(ctx, words, levelWords, levelItems, offsets, 0, s);
 }
 
 // BasicDAG -> snapshot conversion state: one item list per level, memoised by BasicDAG index.

@@ -220,13 +220,12 @@ struct TiledBuild {
     unsigned long long topBytes;
 
     // Allocates the level tables (bottom-up, canonical items first) and makes them current.
-    svdag_status alloc_tables(const std::vector<std::vector<uint32_t>>& buckets, bool provisional, cudaStream_t s)
+    svdag_status alloc_tables(const std::vector<std::vector<uint32_t>>& buckets, uint32_t least, cudaStream_t s)
     {
         const uint32_t LL = ctx->cfg.levels - 2;
         for (int level = (int)LL; level >= 0; --level) {
             svdag_table& t = ctx->levelTables[level];
-            const uint32_t kind = level == (int)LL ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE;
-            SVDAG_TRY(provisional ? alloc_table(ctx, &t, kind, buckets[level].data(), s, true) : alloc_level_table(ctx, &t, kind, buckets[level].data(), s));
+            SVDAG_TRY(alloc_level_table(ctx, &t, level == (int)LL ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets[level].data(), least, s));
             t.level = level;
             SVDAG_TRY(insert_canonical(ctx, (uint32_t)level, s));
         }
@@ -384,7 +383,7 @@ svdag_status run_scene_build(svdag_ctx* ctx, const svdag_terrain_params* p, cuda
     }
     uint32_t root = kNone;
     SVDAG_TRY(reset_dag(ctx, s));
-    SVDAG_TRY(tb.alloc_tables(buckets, true, s));
+    SVDAG_TRY(tb.alloc_tables(buckets, 0, s));
     SVDAG_TRY(tb.build(root, s));
     unsigned long long* counters = reinterpret_cast<unsigned long long*>(tb.top + topBytes - 256);
     for (uint32_t level = 0; level <= LL; ++level) {
@@ -393,10 +392,23 @@ svdag_status run_scene_build(svdag_ctx* ctx, const svdag_terrain_params* p, cuda
         for (uint32_t c = 0; c < kNumClasses; ++c)
             buckets[level][c] = (uint32_t)std::max<unsigned long long>(1, (per[c] + ctx->loadFactor - 1) / ctx->loadFactor);
     }
-    // Final pass into exactly sized tables.
+    // Final pass into tables of the counted size, with the level tables' minimum where it leaves room for the scene.
     SVDAG_TRY(reset_dag(ctx, s));
-    SVDAG_TRY(tb.alloc_tables(buckets, false, s));
-    SVDAG_TRY(tb.build(root, s));
+    TableSpace wanted;
+    for (const auto& b : buckets)
+        wanted.add(b.data());
+    uint32_t least = 0;
+    SVDAG_TRY(level_table_minimum(ctx, wanted, &least, s));
+    auto final_pass = [&](uint32_t minimum) {
+        SVDAG_TRY(tb.alloc_tables(buckets, minimum, s));
+        return tb.build(root, s);
+    };
+    svdag_status st = final_pass(least);
+    if (st == SVDAG_ERR_OOM && least) {
+        SVDAG_TRY(reset_dag(ctx, s));
+        st = final_pass(0);
+    }
+    SVDAG_TRY(st);
     SVDAG_CUDA(cudaMemcpyAsync(&ctx->ctl->root, &root, sizeof(root), cudaMemcpyHostToDevice, s));
     SVDAG_CUDA(cudaStreamSynchronize(s));
     return SVDAG_OK;

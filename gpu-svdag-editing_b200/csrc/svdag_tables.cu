@@ -124,24 +124,37 @@ void reset_level_tables(svdag_ctx* ctx)
         t = svdag_table {};
 }
 
-// Allocates a level table of at least the given bucket counts. Every edit leaves a new version of each node on
+// The least bucket count a class of every level table starts with. Every edit leaves a new version of each node on
 // its path, so the table of an upper level grows with the edits whatever its scene held: sized from
 // the scene alone, the root's table has one bucket of the class all its versions fall in, a group of
 // edits takes turns on that bucket's lock and each one walks its chain. 256 scattered small edits at
 // depth 15 took 5.03 ms that way and 2.79 ms with these tables. 2048 buckets hold 32768 versions at the
-// default load; all levels' minimum together takes at most 1/32 of the region.
-svdag_status alloc_level_table(svdag_ctx* ctx, svdag_table* t, uint32_t kind, const uint32_t* bucketsPerClass, cudaStream_t s)
+// default load; all levels' minimum together takes at most 1/32 of the space that the regions have left after the
+// `wanted` tables. Scenes and snapshots that then do not fit are built once more without it (a minimum of 0).
+svdag_status level_table_minimum(svdag_ctx* ctx, const TableSpace& wanted, uint32_t* least, cudaStream_t s)
 {
-    unsigned long long row = 0; // bytes of one bucket of every class
-    for (uint32_t k = 2; k < 2 + kNumClasses; ++k)
-        row += slab_bytes(k);
-    const unsigned long long region = ctx->itemWords * 4ull + ctx->headerCount * 32ull;
-    const uint32_t least = (uint32_t)std::min<unsigned long long>(2048, region / 32 / (ctx->cfg.levels - 1) / row);
+    unsigned long long tops[2] = { 0, 0 }; // itemTop (words), headerTop (headers)
+    SVDAG_CUDA(cudaMemcpyAsync(tops, &ctx->ctl->itemTop, sizeof(tops), cudaMemcpyDeviceToHost, s));
+    SVDAG_CUDA(cudaStreamSynchronize(s));
+    const unsigned long long words = tops[0] + wanted.words, headers = tops[1] + wanted.headers;
+    const unsigned long long freeWords = ctx->itemWords > words ? ctx->itemWords - words : 0;
+    const unsigned long long freeHeaders = ctx->headerCount > headers ? ctx->headerCount - headers : 0;
+    uint32_t one[kNumClasses];
+    std::fill(one, one + kNumClasses, 1u);
+    TableSpace row; // one bucket of every class
+    row.add(one);
+    const unsigned long long share = 32ull * (ctx->cfg.levels - 1);
+    *least = (uint32_t)std::min({ 2048ull, freeWords / share / row.words, freeHeaders / share / row.headers });
+    return SVDAG_OK;
+}
+
+// Allocates a level table of the given bucket counts, raised to `least`.
+svdag_status alloc_level_table(svdag_ctx* ctx, svdag_table* t, uint32_t kind, const uint32_t* bucketsPerClass, uint32_t least, cudaStream_t s)
+{
     uint32_t buckets[kNumClasses];
     for (uint32_t c = 0; c < kNumClasses; ++c)
         buckets[c] = std::max(bucketsPerClass[c], least);
-    const svdag_status st = alloc_table(ctx, t, kind, buckets, s, true);
-    return st == SVDAG_ERR_OOM ? alloc_table(ctx, t, kind, bucketsPerClass, s, true) : st; // a region that is nearly full
+    return alloc_table(ctx, t, kind, buckets, s, true);
 }
 
 // Default bucket counts for a level that was not sized by a scene build: the surface of a scene
@@ -149,21 +162,31 @@ svdag_status alloc_level_table(svdag_ctx* ctx, svdag_table* t, uint32_t kind, co
 svdag_status ensure_level_tables(svdag_ctx* ctx, cudaStream_t s)
 {
     const uint32_t leaf = ctx->cfg.levels - 2;
+    uint32_t buckets[kMaxLevels][kNumClasses];
+    TableSpace wanted;
     bool created = false;
+    for (uint32_t level = 0; level <= leaf; ++level) {
+        if (ctx->levelTables[level].ready)
+            continue;
+        const unsigned long long expect = std::min<unsigned long long>(1ull << (2 * (level + 1)), 1ull << 20);
+        for (uint32_t c = 0; c < kNumClasses; ++c)
+            buckets[level][c] = (uint32_t)std::max<unsigned long long>(1, expect / (4ull * ctx->loadFactor));
+        wanted.add(buckets[level]);
+        created = true;
+    }
+    if (!created)
+        return SVDAG_OK;
+    uint32_t least = 0;
+    SVDAG_TRY(level_table_minimum(ctx, wanted, &least, s));
     for (int level = (int)leaf; level >= 0; --level) {
         svdag_table& t = ctx->levelTables[level];
         if (t.ready)
             continue;
-        const unsigned long long expect = std::min<unsigned long long>(1ull << (2 * (level + 1)), 1ull << 20);
-        uint32_t buckets[kNumClasses];
-        for (uint32_t c = 0; c < kNumClasses; ++c)
-            buckets[c] = (uint32_t)std::max<unsigned long long>(1, expect / (4ull * ctx->loadFactor));
-        SVDAG_TRY(alloc_level_table(ctx, &t, level == (int)leaf ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets, s));
+        SVDAG_TRY(alloc_level_table(ctx, &t, level == (int)leaf ? SVDAG_KIND_LEAF : SVDAG_KIND_NODE, buckets[level], least, s));
         t.level = level;
         SVDAG_TRY(insert_canonical(ctx, (uint32_t)level, s));
-        created = true;
     }
-    return created ? upload_tables(ctx, s) : SVDAG_OK;
+    return upload_tables(ctx, s);
 }
 
 svdag_status upload_tables(svdag_ctx* ctx, cudaStream_t s)
