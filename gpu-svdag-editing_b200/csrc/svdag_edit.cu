@@ -2362,15 +2362,19 @@ constexpr unsigned long long kSubtreeScratch = 16ull << 20; // scratch slice of 
 // Launches expanded editors with their editors and records in `region`: an edit as its chain of
 // launches, or a run of small edits whose nodes are pairwise disjoint as one group (one block per edit
 // builds its subtree, then the paths from the root to the subtrees are rebuilt and committed in order:
-// k_edit_subtrees, k_edit_spines), where that is the faster of the two. Measured for spheres and boxes
-// at depth 14: a chain takes 55 us and 5 us more per 1000 estimated leaves (radius 9: 68, radius 70: 113);
-// a group takes 60 us for its paths and its slowest block, which is 55 us and 35 us more per 1000
-// leaves (radius 20: 90, radius 70: 390-590). An edit alone runs in the one-block kernel, where the context
-// asks for it, only up to 400 leaves, where one launch takes what the chain takes (radius 9: 68 against
-// 68 us; radius 20: 92 against 80, radius 45: 200 against 98).
+// k_edit_subtrees, k_edit_spines), where that is the faster of the two by the costs below. They are fits over the
+// six tools that form groups, radii 2 to 60, 2 to 100 edits and depths 9, 12, 14 and 17 (876 batches, run as chains and as one
+// group). A chain by depth and leaves: radius 2 at depth 9 44 us, at depth 17 70; radius 60 92 and 128. A group by its paths, its
+// edits and its slowest block: 8 edits of radius 2 at depth 9 71 us, at depth 17 91; of radius 60 at depth 17 252. The fit gives a
+// block 18 us per 1000 leaves, 30 are charged: paints of solid ground take up to twice the fit (128 of radius 60 at depth 12: 49.5 ms
+// in the groups that 18 chooses, 30.9 in those of 30), and elsewhere both choose alike (704 batches of all tools: 5.6 and 5.5 %
+// less time than with costs fitted to spheres and boxes at depth 14 alone, where 8 mixed edits of radii up to 60 took 1.7 times
+// their group's time). An edit alone
+// runs in the one-block kernel, where the context asks for it, only up to 400 leaves, where one launch takes what the chain takes
+// (radius 9: 68 against 68 us; radius 20: 92 against 80, radius 45: 200 against 98).
 constexpr double kBlockAloneLeaves = 400.0;
-double chain_us(double leaves) { return 55.0 + 0.005 * leaves; }
-double group_us(double mostLeaves) { return 60.0 + 55.0 + 0.035 * mostLeaves; }
+double chain_us(uint32_t levels, double leaves) { return 7.0 + 3.25 * levels + 6.5 * std::log2(1.0 + leaves / 100.0); }
+double group_us(uint32_t levels, uint32_t edits, double mostLeaves) { return 25.0 + 2.75 * levels + 2.2 * edits + 0.03 * mostLeaves; }
 
 svdag_status launch_edits_at(svdag_ctx* ctx, const DevEditor* eds, uint32_t n, char* region, size_t regionBytes, cudaStream_t s)
 {
@@ -2419,10 +2423,11 @@ svdag_status launch_edits_at(svdag_ctx* ctx, const DevEditor* eds, uint32_t n, c
         double chains = 0, most = 0, best = 0;
         for (uint32_t q = k; q < e; ++q) {
             const double leaves = estimate_leaves(eds[q]);
-            chains += chain_us(leaves);
+            chains += chain_us(ctx->cfg.levels, leaves);
             most = std::max(most, leaves);
-            if (chains - group_us(most) > best) {
-                best = chains - group_us(most);
+            const double gain = chains - group_us(ctx->cfg.levels, q + 1 - k, most);
+            if (gain > best) {
+                best = gain;
                 m = q + 1 - k;
             }
         }
