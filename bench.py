@@ -928,9 +928,9 @@ def run_mode_trace(args):
 
 
 def c3_compare(svdag, w, torch, levels, edits):
-    """The edits through the plain per-edit path and through one batch (the persistent kernel for small
-    edits, subtree groups for runs of small edits in disjoint nodes), each on its own copy of the
-    scene; the stored item sets must be equal."""
+    """The edits through the plain per-edit path and through one batch (subtree groups for runs of small
+    edits in disjoint nodes, chains of launches for the others), each on its own copy of the scene; the
+    stored item sets must be equal."""
     res, items = {}, {}
     for name in ("plain", "batched"):
         dag, _ = make_scene(svdag, w, levels, persistent=name == "batched")
@@ -987,7 +987,7 @@ def main():
     ap.add_argument("--sweep", default="50,200,500,2000", help="other offered loads (edits/s) served and plain")
     ap.add_argument("--levels", type=int, default=17)
     ap.add_argument("--phase-kernels", action="store_true", help="one launch per edit phase (profiling)")
-    ap.add_argument("--persistent", action="store_true", help="small edits in the persistent cooperative kernel")
+    ap.add_argument("--persistent", action="store_true", help="small edits alone in one block, or grouped in a batch")
     ap.add_argument("--pool-gb", type=float, default=0.0, help="pool size of the c2 mode's scene (0 = by depth)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-hash", action="store_true")

@@ -1794,10 +1794,10 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_edit_bottom(DevDag d, uint
 }
 
 // ---------------------------------------------------------------- persistent form
-// The persistent form for small edits: one CTA of 512 threads runs whole edits, one after another:
-// the narrow levels as above, the others as block-stride loops over the device-resident counts, the
-// phases separated by block barriers. Small SVOs thus cost one launch per batch. All threads reach every
-// barrier (phases only return early, never skip a barrier).
+// The persistent form for small edits: one CTA of 512 threads runs a whole edit: the narrow levels as
+// above, the others as block-stride loops over the device-resident counts, the phases separated by block
+// barriers. A small edit alone is one launch (k_edit_block), a group of them one block each
+// (k_edit_subtrees). All threads reach every barrier (phases only return early, never skip a barrier).
 
 // Top-down phases and the leaves; returns the first level that narrow_build left.
 template <uint32_t TOOL>
@@ -1820,7 +1820,7 @@ __device__ __forceinline__ uint32_t block_build(const DevDag& d, const DevEditor
 // One whole edit in this block. SUBTREES: an edit of a group (the tools that qualify, shared tables).
 template <bool SUBTREES>
 __device__ __forceinline__ void block_edit(const DevDag& d, const DevEditor& ed, char* scratch, unsigned long long scratchBytes,
-    EditRecord* record, NarrowShared& sh)
+    NarrowShared& sh)
 {
     const uint32_t LL = d.leafLevel;
     uint32_t k = 0, wide = LL;
@@ -1872,7 +1872,7 @@ __device__ __forceinline__ void block_edit(const DevDag& d, const DevEditor& ed,
     else if (merge_live(d))
         root = merged_top(d, scratch);
     if (threadIdx.x == 0)
-        edit_end(d, root, ed.builder, ed.tileOut, record);
+        edit_end(d, root, ed.builder, ed.tileOut, nullptr); // a group's records are k_edit_spines'
     __syncthreads();
     stamp(d, k);
 }
@@ -1886,15 +1886,13 @@ __device__ __forceinline__ void load_editor(DevEditor& to, const DevEditor& from
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kBlockThreads, 1) k_edit_block(DevDag d, const __grid_constant__ DevEditor single, const DevEditor* eds,
-    uint32_t numEdits, char* scratch, unsigned long long scratchBytes, EditRecord* records)
+__global__ void __launch_bounds__(kBlockThreads, 1) k_edit_block(DevDag d, const __grid_constant__ DevEditor editor, char* scratch,
+    unsigned long long scratchBytes)
 {
     __shared__ NarrowShared sh;
     __shared__ DevEditor ed;
-    for (uint32_t k = 0; k < numEdits; ++k) {
-        load_editor(ed, eds ? eds[k] : single);
-        block_edit<false>(d, ed, scratch, scratchBytes, records ? &records[k] : nullptr, sh);
-    }
+    load_editor(ed, editor);
+    block_edit<false>(d, ed, scratch, scratchBytes, sh);
 }
 
 // A group of subtree edits (DevEditor::subtree) whose nodes are pairwise disjoint: block k builds and
@@ -1914,7 +1912,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_edit_subtrees(DevDag d, co
     dk.solo = 1;
     __shared__ DevEditor ed;
     load_editor(ed, eds[k]);
-    block_edit<true>(dk, ed, parts + (unsigned long long)k * partBytes, partBytes, nullptr, sh);
+    block_edit<true>(dk, ed, parts + (unsigned long long)k * partBytes, partBytes, sh);
 }
 
 // Commits a group of subtree edits: each edit's path from its node up to the root (levels
@@ -2508,7 +2506,7 @@ int expand_edit(const svdag_ctx* ctx, const svdag_edit& e, DevEditor* out)
 // One small edit as one persistent launch, its editor passed by value.
 svdag_status launch_single_fused(svdag_ctx* ctx, const DevEditor& ed, cudaStream_t s)
 {
-    k_edit_block<<<1, kBlockThreads, 0, s>>>(ctx->dag(), ed, nullptr, 1, ctx->scratch, ctx->scratchBytes, nullptr);
+    k_edit_block<<<1, kBlockThreads, 0, s>>>(ctx->dag(), ed, ctx->scratch, ctx->scratchBytes);
     SVDAG_CUDA(cudaGetLastError());
     return SVDAG_OK;
 }
@@ -2624,11 +2622,11 @@ svdag_status build_scene_untiled(svdag_ctx* ctx, const DevEditor& ed, cudaStream
     return build_scene_untiled_into(ctx, ed, 0, sized, s);
 }
 
-// Tiles of a scene: every tile is a builder edit of the subtree under one node, all tiles of a call
-// in one persistent launch (the level tables exist already; the merge phase finds or inserts).
+// Tiles of a scene: every tile is a builder edit of the subtree under one node (the level tables exist
+// already; the merge phase finds or inserts).
 svdag_status launch_scene_tiles(svdag_ctx* ctx, const DevEditor* eds, uint32_t n, cudaStream_t s)
 {
-    for (uint32_t i = 0; i < n; ++i) // tiles are large: one launch per phase at full occupancy
+    for (uint32_t i = 0; i < n; ++i) // tiles are large: a chain of launches each
         SVDAG_TRY(launch_pipeline(ctx, eds[i], s, nullptr));
     return SVDAG_OK;
 }

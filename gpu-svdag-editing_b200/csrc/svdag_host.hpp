@@ -25,7 +25,7 @@ struct svdag_ctx {
     svdag::Control* ctl = nullptr; // device control block
     char* scratch = nullptr; // per-edit arena
     unsigned long long scratchBytes = 0;
-    char* batch = nullptr; // editors and per-edit records of a persistent batch launch
+    char* batch = nullptr; // editors and per-edit records of a batch
     unsigned long long batchBytes = 0;
     uint32_t lastBatch = 0;
     uint32_t* items = nullptr; // item region
@@ -35,7 +35,7 @@ struct svdag_ctx {
     svdag_table levelTables[svdag::kMaxLevels];
     std::vector<svdag_table*> standalone;
     uint32_t probeLanes = 8;
-    double persistentLeaves = 0; // edits estimated at or below this many SVO leaves run in the persistent kernel (0 = none)
+    double persistentLeaves = 0; // edits estimated at or below this many SVO leaves may be grouped in a batch and, up to 400, run alone in one block (0 = none)
     uint32_t loadFactor = 16;
     unsigned long long scratchHighWater = 0;
     svdag::DevDag dag() const { return svdag::DevDag { items, itemWords, headers, headerCount, ctl, cfg.levels, cfg.levels - 2, &ctl->edit, 0u, nullptr }; }
@@ -117,8 +117,8 @@ svdag_status reset_dag(svdag_ctx* ctx, cudaStream_t s);
 svdag_status build_scene_untiled(svdag_ctx* ctx, const DevEditor& ed, cudaStream_t s);
 // Builds the subtrees of scene tiles, one builder editor per tile (svdag_edit.cu).
 svdag_status launch_scene_tiles(svdag_ctx* ctx, const DevEditor* eds, uint32_t n, cudaStream_t s);
-// Edit validation, expansion into device editors (a move gives two) and the persistent launch of
-// expanded editors with their editors and records in `region` (svdag_edit.cu).
+// Edit validation, expansion into device editors (a move gives two), the one-block and the chained launch of one
+// editor (svdag_edit.cu; launch_edits_at below takes a batch of them, with editors and records in `region`).
 bool valid_edit(const svdag_edit* e);
 int expand_edit(const svdag_ctx* ctx, const svdag_edit& e, DevEditor* out);
 double estimate_leaves(const DevEditor& e);

@@ -444,7 +444,7 @@ class MyGPUHashDAG:
         _check(lib().svdag_edit_apply(self.h, C.byref(e), stream_ptr(stream)), "svdag_edit_apply")
 
     def edit_batch(self, editors, stream=None) -> int:
-        """Batched form: all edits in one persistent launch. Returns the number of records
+        """Batched form: groups of small edits side by side, the others as chains of launches. Returns the number of records
         (a move yields two)."""
         arr = (Edit * len(editors))(*[e if isinstance(e, Edit) else e.to_edit() for e in editors])
         _check(lib().svdag_edit_apply_many(self.h, arr, len(editors), stream_ptr(stream)), "svdag_edit_apply_many")
@@ -514,7 +514,7 @@ class MyGPUHashDAG:
 
     def autotune(self, edits=(), keys=None, offsets=None, n_keys=0, total_words=0, kind=0, stream=None) -> "Tuning":
         """Autotuner (svdag_autotune): key sample -> load factor and lanes per key; edit sample (applied
-        for real) -> which small edits use the persistent kernel."""
+        for real) -> which small edits a batch may group (and run alone in one block)."""
         arr = (Edit * max(len(edits), 1))(*[e if isinstance(e, Edit) else e.to_edit() for e in edits])
         t = Tuning()
         _check(lib().svdag_autotune(self.h, arr, len(edits), ptr(keys), ptr(offsets), n_keys, total_words, kind,
