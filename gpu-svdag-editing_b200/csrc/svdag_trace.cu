@@ -148,7 +148,9 @@ __device__ __forceinline__ bool ray_meets_box(const RayF& r, const float* b)
 
 // intersect_ray, tracer.cu:186-273: the first voxel on the ray and its material; leaves the coordinates as they
 // are when there is none. Stack in shared memory, [level][thread] so that a warp's accesses hit distinct
-// banks. Bound by the integer and compare pipe (75 % busy).
+// banks. At 1920x1080 and depth 14 the integer and compare pipe is 60 % busy, 22 of 32 lanes are active and the
+// longest stall is the wait for a node (71 % of them in L1). The form of the tests that any_hit has for rays without
+// NaN gains nothing here (33x17 to 1920x1080: 0.5 to 2 % more time with both forms in the kernel).
 __device__ __forceinline__ void first_hit(const DevDag& d, uint32_t root, const RayF& r, uint32_t (*sIndex)[256], uint32_t (*sMasks)[256],
     const uint8_t* sNext, uint32_t tix, uint32_t& px, uint32_t& py, uint32_t& pz, uint32_t& material)
 {
