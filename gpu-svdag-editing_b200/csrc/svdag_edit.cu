@@ -1773,7 +1773,7 @@ __global__ void __launch_bounds__(256, 4) k_merge_level(DevDag d, uint32_t level
     ph_merge_level<false>(d, level, scratch);
 }
 template <int G>
-__global__ void __launch_bounds__(256) k_insert_level(DevDag d, DevTable t, uint32_t level, char* scratch)
+__global__ void __launch_bounds__(256) k_insert_level(const __grid_constant__ DevDag d, const __grid_constant__ DevTable t, uint32_t level, char* scratch)
 {
     ph_insert_level<G>(d, t, level, scratch);
 }

@@ -211,7 +211,8 @@ enum { OP_FIND = 0, OP_ADD = 1, OP_FIND_OR_INSERT = 2 };
 // them wait for memory, so warps in flight count for more than a few spills of the rare paths (adds of 2^21 keys
 // at 16 a bucket with 32 lanes a key: 617 us with 32 registers, 866 with 40; with 16: 413 and 550); lower caps on one
 // lane's add cost 10 to 24 %. A lookup with 32 lanes has no cap (2^22 keys at 96 a bucket: 2329 us without, 2560
-// with).
+// with). The DAG is a grid constant: the out-of-line inserts take it by reference, which would otherwise put a copy of it on
+// every thread's stack (65536 keys that are all there, 8 a bucket, 4 to 16 lanes: 46 to 54 us with the copy, 42 to 50 without).
 template <int G, int OP>
 constexpr int table_op_blocks()
 {
@@ -219,7 +220,7 @@ constexpr int table_op_blocks()
 }
 
 template <int G, int OP>
-__global__ void __launch_bounds__(256, table_op_blocks<G, OP>()) k_table_op(DevDag d, DevTable t, const uint32_t* __restrict__ keys,
+__global__ void __launch_bounds__(256, table_op_blocks<G, OP>()) k_table_op(const __grid_constant__ DevDag d, DevTable t, const uint32_t* __restrict__ keys,
     const uint32_t* __restrict__ offsets, uint32_t n, unsigned long long totalWords, const uint32_t* __restrict__ reps,
     uint32_t* __restrict__ out)
 {
