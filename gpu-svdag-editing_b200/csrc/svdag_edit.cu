@@ -2612,8 +2612,7 @@ static svdag_status build_scene_untiled_into(svdag_ctx* ctx, const DevEditor& ed
 svdag_status build_scene_untiled(svdag_ctx* ctx, const DevEditor& ed, cudaStream_t s)
 {
     SVDAG_TRY(reset_dag(ctx, s));
-    uint32_t least = 0;
-    SVDAG_TRY(level_table_minimum(ctx, TableSpace {}, &least, s));
+    const uint32_t least = level_table_minimum(ctx, kFreshRegions, TableSpace {});
     bool sized = false;
     const svdag_status st = build_scene_untiled_into(ctx, ed, least, sized, s);
     if (st != SVDAG_ERR_OOM || !sized || !least)

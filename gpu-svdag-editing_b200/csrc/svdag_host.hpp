@@ -99,7 +99,8 @@ struct TableSpace {
         }
     }
 };
-svdag_status level_table_minimum(svdag_ctx* ctx, const TableSpace& wanted, uint32_t* least, cudaStream_t s);
+uint32_t level_table_minimum(const svdag_ctx* ctx, const TableSpace& used, const TableSpace& wanted);
+constexpr TableSpace kFreshRegions { 0, 1 }; // after reset_dag (header 0 is never used)
 svdag_status alloc_level_table(svdag_ctx* ctx, svdag_table* t, uint32_t kind, const uint32_t* bucketsPerClass, uint32_t least, cudaStream_t s);
 // Find-or-insert of keys that are pairwise distinct (no batch dedup) into a level table.
 svdag_status find_or_insert_distinct(svdag_ctx* ctx, uint32_t level, const uint32_t* keys, const uint32_t* offsets, uint32_t n,

@@ -178,8 +178,7 @@ svdag_status load_snapshot(svdag_ctx* ctx, const uint32_t* words, const uint64_t
         base += levelWords[level];
     }
     SVDAG_TRY(reset_dag(ctx, s));
-    uint32_t least = 0;
-    SVDAG_TRY(level_table_minimum(ctx, wanted, &least, s));
+    const uint32_t least = level_table_minimum(ctx, kFreshRegions, wanted);
     const svdag_status st = load_snapshot_into(ctx, words, levelWords, levelItems, offsets, least, s);
     if (st != SVDAG_ERR_OOM || !least)
         return st;

@@ -397,8 +397,7 @@ svdag_status run_scene_build(svdag_ctx* ctx, const svdag_terrain_params* p, cuda
     TableSpace wanted;
     for (const auto& b : buckets)
         wanted.add(b.data());
-    uint32_t least = 0;
-    SVDAG_TRY(level_table_minimum(ctx, wanted, &least, s));
+    const uint32_t least = level_table_minimum(ctx, kFreshRegions, wanted);
     auto final_pass = [&](uint32_t minimum) {
         SVDAG_TRY(tb.alloc_tables(buckets, minimum, s));
         return tb.build(root, s);

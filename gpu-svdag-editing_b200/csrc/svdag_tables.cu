@@ -131,12 +131,10 @@ void reset_level_tables(svdag_ctx* ctx)
 // depth 15 took 5.03 ms that way and 2.79 ms with these tables. 2048 buckets hold 32768 versions at the
 // default load; all levels' minimum together takes at most 1/32 of the space that the regions have left after the
 // `wanted` tables. Scenes and snapshots that then do not fit are built once more without it (a minimum of 0).
-svdag_status level_table_minimum(svdag_ctx* ctx, const TableSpace& wanted, uint32_t* least, cudaStream_t s)
+// `used`: what the bump pointers have handed out.
+uint32_t level_table_minimum(const svdag_ctx* ctx, const TableSpace& used, const TableSpace& wanted)
 {
-    unsigned long long tops[2] = { 0, 0 }; // itemTop (words), headerTop (headers)
-    SVDAG_CUDA(cudaMemcpyAsync(tops, &ctx->ctl->itemTop, sizeof(tops), cudaMemcpyDeviceToHost, s));
-    SVDAG_CUDA(cudaStreamSynchronize(s));
-    const unsigned long long words = tops[0] + wanted.words, headers = tops[1] + wanted.headers;
+    const unsigned long long words = used.words + wanted.words, headers = used.headers + wanted.headers;
     const unsigned long long freeWords = ctx->itemWords > words ? ctx->itemWords - words : 0;
     const unsigned long long freeHeaders = ctx->headerCount > headers ? ctx->headerCount - headers : 0;
     uint32_t one[kNumClasses];
@@ -144,8 +142,7 @@ svdag_status level_table_minimum(svdag_ctx* ctx, const TableSpace& wanted, uint3
     TableSpace row; // one bucket of every class
     row.add(one);
     const unsigned long long share = 32ull * (ctx->cfg.levels - 1);
-    *least = (uint32_t)std::min({ 2048ull, freeWords / share / row.words, freeHeaders / share / row.headers });
-    return SVDAG_OK;
+    return (uint32_t)std::min({ 2048ull, freeWords / share / row.words, freeHeaders / share / row.headers });
 }
 
 // Allocates a level table of the given bucket counts, raised to `least`.
@@ -176,8 +173,10 @@ svdag_status ensure_level_tables(svdag_ctx* ctx, cudaStream_t s)
     }
     if (!created)
         return SVDAG_OK;
-    uint32_t least = 0;
-    SVDAG_TRY(level_table_minimum(ctx, wanted, &least, s));
+    unsigned long long tops[2] = { 0, 0 }; // itemTop (words), headerTop (headers)
+    SVDAG_CUDA(cudaMemcpyAsync(tops, &ctx->ctl->itemTop, sizeof(tops), cudaMemcpyDeviceToHost, s));
+    SVDAG_CUDA(cudaStreamSynchronize(s));
+    const uint32_t least = level_table_minimum(ctx, TableSpace { tops[0], tops[1] }, wanted);
     for (int level = (int)leaf; level >= 0; --level) {
         svdag_table& t = ctx->levelTables[level];
         if (t.ready)
